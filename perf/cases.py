@@ -185,6 +185,121 @@ def work(case):
     return {"bytes": NL * layer_bytes + V * H * 2 + T * H * 2 + B * V * 4, "flops": NL * layer_flops + 2.0 * B * V * H}
 
 
+def _unpack_q4k(raw, shape):
+    """Q4_K bytes -> the values they stand for, f64: d*scale*q - dmin*min, (scale, min) six bits each."""
+    blk = raw.view(-1, 144)
+    d, dmin = blk[:, 0:4].contiguous().view(torch.float16).double().split(1, 1)
+    lo, mid, hi = blk[:, 4:8].int(), blk[:, 8:12].int(), blk[:, 12:16].int()
+    sc = torch.cat([lo & 63, (hi & 15) | ((lo >> 6) << 4)], 1).double()
+    mn = torch.cat([mid & 63, (hi >> 4) | ((mid >> 6) << 4)], 1).double()
+    q = blk[:, 16:].view(-1, 4, 32)
+    q = torch.stack([q & 15, q >> 4], 2).view(-1, 8, 32).double()
+    return ((d * sc)[:, :, None] * q - (dmin * mn)[:, :, None]).view(shape)
+
+
+def _moe64(x, router, bias, banks, shapes, top_k, norm):
+    """The layer in 64 bits from the values its weights stand for; banks as given to the handle, one expert at a time."""
+    p = torch.softmax(x @ router + bias, -1)
+    w, ids = p.topk(top_k, -1)
+    if norm:
+        w = w / w.sum(-1, keepdim=True)
+    y = torch.zeros_like(x)
+
+    def weight(b, e):
+        if banks[b].dtype == torch.uint8:
+            return _unpack_q4k(banks[b].view(shapes[b][0], -1)[e], shapes[b][1:])
+        return banks[b][e].double()
+    for e in range(shapes[0][0]):
+        t, k = (ids == e).nonzero(as_tuple=True)
+        if t.numel():
+            h = torch.nn.functional.silu(x[t] @ weight(0, e).T) * (x[t] @ weight(1, e).T)
+            y[t] += (h @ weight(2, e).T) * w[t, k][:, None]
+    return y
+
+
+def _exact_layers(case, gen):
+    H, I, E = case["hidden"], case["inter"], case["experts"]
+    shapes = [(E, I, H), (E, I, H), (E, H, I)]
+    bias = synth.zipf_router_bias(E, case["skew"]) if case["skew"] else [0.0] * E
+    bias = torch.tensor(bias, dtype=torch.float64, device="cuda")
+    layers = []
+    for _ in range(case["layers"]):
+        router = (torch.randn(H, E, generator=gen, device="cuda") * 0.02).double()
+        banks = []
+        for shape in shapes:
+            w = torch.randn(shape, generator=gen, device="cuda").mul_(0.02)
+            banks.append(moe.q4k_quantize_device(w) if case["dtype"] == "q4_k" else w.to(TORCH[case["dtype"]]))
+        layers.append((router, banks))
+    xs = [torch.randn(case["tokens"], H, generator=gen, device="cuda").to(TORCH[case["dtype"]]).double() for _ in layers]
+    return [_moe64(x, r, bias, b, shapes, case["top_k"], case["norm"]) for x, (r, b) in zip(xs, layers)]
+
+
+def _exact_model(case, gen, seed):
+    """The decoder in 64 bits from the 16-bit and packed weights: new tokens against a cache (decode) or against each
+    other (prompt).  The weights are drawn as `OlmoeDecoder.random_init` draws them."""
+    c = OlmoeConfig()
+    H, E, I, V, NL, nh, hd = (c.hidden_size, c.num_experts, c.intermediate_size, c.vocab_size, c.num_hidden_layers,
+                              c.num_attention_heads, c.head_dim)
+    B = case["batch"]
+    decode = case["kind"] == "decode"
+    keys = case["keys"] if decode else case["length"]
+    ids = torch.randint(0, V, (B, keys), generator=gen, device="cuda")
+    lengths = [0] * B
+    if decode:
+        kc, vc = (torch.empty(NL, B, nh, 640, hd, dtype=torch.float16, device="cuda") for _ in range(2))
+        kc.normal_(generator=gen)
+        vc.normal_(generator=gen).mul_(0.9)
+        lengths = [keys - (7 * b) % (keys // 4 + 1) for b in range(B)]
+        ids = ids[:, -1:]
+    T = ids.shape[1]
+    wgen = torch.Generator(device="cuda")
+    wgen.manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, generator=wgen, device="cuda") * 0.02
+    embed, lm_head = rnd(V, H).to(torch.float16).mul_(50.0), rnd(V, H).to(torch.float16)
+    shapes = [(E, I, H), (E, I, H), (E, H, I)]
+    rms = lambda v: v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + c.rms_norm_eps)
+    pos = torch.tensor(lengths, device="cuda")[:, None] + torch.arange(T, device="cuda")
+    half = torch.arange(hd // 2, device="cuda", dtype=torch.float64)
+    ang = (pos[..., None] * c.rope_theta ** (-2.0 * half / hd))[:, None]                 # [B, 1, T, hd / 2]
+    cos, sin = torch.cat([ang.cos()] * 2, -1), torch.cat([ang.sin()] * 2, -1)
+    rope = lambda v: v * cos + torch.cat([-v[..., hd // 2:], v[..., :hd // 2]], -1) * sin
+    heads = lambda v: v.view(B, T, nh, hd).transpose(1, 2)
+    x = embed[ids].double()
+    ks, vs = [], []
+    for l in range(NL):
+        wq, wk, wv, wo = (rnd(H, H).to(torch.float16).double() for _ in range(4))
+        router = rnd(H, E).double()
+        banks = [moe.q4k_quantize_device(rnd(*shape)) for shape in shapes]
+        h = rms(x)
+        q, k, v = rope(heads(rms(h @ wq.T))), rope(heads(rms(h @ wk.T))), heads(h @ wv.T)
+        out = torch.empty_like(q)
+        for b in range(B):
+            kb, vb = k[b], v[b]
+            if decode:
+                kb = torch.cat([kc[l, b, :, :lengths[b]].double(), kb], 1)
+                vb = torch.cat([vc[l, b, :, :lengths[b]].double(), vb], 1)
+            score = q[b] @ kb.transpose(1, 2) / math.sqrt(hd)
+            late = torch.arange(kb.shape[1], device="cuda")[None, :] > pos[b][:, None]
+            out[b] = torch.softmax(score.masked_fill(late, -math.inf), -1) @ vb
+        x = x + out.transpose(1, 2).reshape(B, T, H) @ wo.T
+        moe_in = rms(x).reshape(B * T, H)
+        x = x + _moe64(moe_in, router, 0.0, banks, shapes, c.num_experts_per_tok, c.norm_topk_prob).view(B, T, H)
+        if not decode:
+            ks.append(k.float())
+            vs.append(v.float())
+    logits = rms(x[:, -1]) @ lm_head.double().T
+    return logits if decode else (logits, torch.stack(ks), torch.stack(vs))
+
+
+def exact(case, seed):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(seed)
+    if case["kind"] in ("layer", "host"):
+        ys = _exact_layers(case, gen)
+        return [y.cpu().numpy() for y in ys] if case["kind"] == "host" else ys
+    return _exact_model(case, gen, seed)
+
+
 def tolerance(case):
     # About four times what was measured (relative 2-norm).  Layers against the same layer in 64 bits from the
     # dequantised weights: 8.5e-4 for packed experts (16-bit intermediate and sub-block sums), 5e-4 for f16, 2.9e-3
