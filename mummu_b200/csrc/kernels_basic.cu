@@ -12,6 +12,7 @@
 #include <cfloat>
 #include <climits>
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tma.cuh"
@@ -1678,6 +1679,131 @@ __global__ void __launch_bounds__(256) simt_grouped_kernel(SimtArgs a) {
     }
 }
 
+// f32 weights with few rows per expert (a decode batch at the reference's own precision): the bank is
+// read once and DRAM is the bound, so the weights stream through shared memory (cp.async, FS_STAGES
+// stages of 128 weight rows x 64 k) and a thread owns one weight row for up to R token rows.  The
+// 64 x 64 tile above keeps 3/4 of its threads on empty rows there and waits for every k slice.
+// Measured, OLMoE shape with 16 tokens (2 rows per expert, 56 experts, 1.41 GB): gate/up 885 -> 183 us
+// (5.1 TB/s), down 503 -> 96 us (4.9 TB/s).
+// A sum is the same ascending chain of FMAs as in the tile kernel: the same bits, whichever ran.
+constexpr int FS_BK = 64, FS_ROWS = 128, FS_STAGES = 3, FS_PITCH = FS_BK + 4;
+
+template <int R>
+constexpr size_t fs_smem_bytes() { return (size_t)FS_STAGES * (FS_ROWS * FS_PITCH + R * FS_BK) * 4; }
+
+template <int R, bool GATEUP>
+__global__ void __launch_bounds__(FS_ROWS) f32_stream_kernel(SimtArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float* ws = reinterpret_cast<float*>(smem_raw);                   // [FS_STAGES][128 weight rows][FS_PITCH]
+    float* xs = ws + FS_STAGES * FS_ROWS * FS_PITCH;                  // [FS_STAGES][R][FS_BK]
+    const int e = a.expert_single >= 0 ? a.expert_single : (int)blockIdx.z;
+    const int cnt = a.counts ? a.counts[e] : a.rows_single;
+    const int m0 = blockIdx.y * R;
+    if (m0 >= cnt) return;
+    const int rn = min(R, cnt - m0);
+    const int base = a.offsets ? a.offsets[e] : 0;
+    const int tid = threadIdx.x;
+    // weight row of tile row t: gate/up: gate n0 + t, up n0 + t - 64; down: n0 + t
+    const int n0 = blockIdx.x * (GATEUP ? 64 : 128);
+    const uint8_t* w0 = a.W0 + (size_t)e * a.expert_stride;
+    const uint8_t* w1 = GATEUP ? a.W1 + (size_t)e * a.expert_stride : w0;
+    const float* A = reinterpret_cast<const float*>(a.A);
+    const int lr = tid >> 4, lc = (tid & 15) * 4;                     // staging: 8 rows x 16 pieces of 16 bytes at a time
+    const float* xrow[(R + 7) / 8];
+#pragma unroll
+    for (int i = 0; i < (R + 7) / 8; ++i) {
+        const int r = lr + 8 * i;
+        const int64_t p = base + m0 + (r < rn ? r : 0);
+        xrow[i] = A + (a.row_index ? (int64_t)a.row_index[p] : p) * a.lda;
+    }
+    const int chunks = (a.K + FS_BK - 1) / FS_BK;
+    auto stage = [&](int c) {
+        if (c < chunks) {
+            const int k = c * FS_BK + lc;
+            float* dw = ws + (size_t)(c % FS_STAGES) * FS_ROWS * FS_PITCH + lc;
+#pragma unroll
+            for (int i = 0; i < FS_ROWS / 8; ++i) {
+                const int t = lr + 8 * i;
+                const int n = n0 + (GATEUP ? (t & 63) : t);
+                const bool ok = n < a.N && k < a.K;
+                const uint8_t* w = (GATEUP && t >= 64) ? w1 : w0;
+                cp_async16_zfill(dw + t * FS_PITCH, w + (ok ? (size_t)n * a.row_bytes + (size_t)k * 4 : 0), ok);
+            }
+            float* dx = xs + (size_t)(c % FS_STAGES) * R * FS_BK + lc;
+#pragma unroll
+            for (int i = 0; i < (R + 7) / 8; ++i) {
+                const int r = lr + 8 * i;
+                const bool ok = r < rn && k < a.K;
+                if (r < R) cp_async16_zfill(dx + r * FS_BK, xrow[i] + (ok ? k : 0), ok);
+            }
+        }
+        cp_async_commit();
+    };
+    float acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < FS_STAGES - 1; ++c) stage(c);
+    for (int c = 0; c < chunks; ++c) {
+        cp_async_wait<FS_STAGES - 2>();
+        __syncthreads();                                              // chunk c has landed; chunk c - 1 is used up
+        stage(c + FS_STAGES - 1);
+        const float* wr = ws + (size_t)(c % FS_STAGES) * FS_ROWS * FS_PITCH + tid * FS_PITCH;
+        const float* xr = xs + (size_t)(c % FS_STAGES) * R * FS_BK;
+#pragma unroll 4
+        for (int k = 0; k < FS_BK; k += 4) {
+            const float4 w = *reinterpret_cast<const float4*>(wr + k);
+#pragma unroll
+            for (int r0 = 0; r0 < R; r0 += 4)
+                if (r0 < rn)
+#pragma unroll
+                    for (int r = r0; r < r0 + 4; ++r) {
+                        const float4 x = *reinterpret_cast<const float4*>(xr + r * FS_BK + k);
+                        acc[r] = fmaf(x.x, w.x, acc[r]);
+                        acc[r] = fmaf(x.y, w.y, acc[r]);
+                        acc[r] = fmaf(x.z, w.z, acc[r]);
+                        acc[r] = fmaf(x.w, w.w, acc[r]);
+                    }
+        }
+    }
+    float* out = reinterpret_cast<float*>(a.out);
+    if constexpr (GATEUP) {
+        float* up = xs;                                               // [R][64]
+        __syncthreads();
+        if (tid >= 64)
+#pragma unroll
+            for (int r = 0; r < R; ++r) up[r * 64 + tid - 64] = acc[r];
+        __syncthreads();
+        if (tid < 64 && n0 + tid < a.N)
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (r < rn) out[(size_t)(base + m0 + r) * a.ldo + n0 + tid] = silu_f(acc[r]) * up[r * 64 + tid];
+    } else {
+        if (n0 + tid < a.N)
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (r < rn) out[(size_t)(base + m0 + r) * a.ldo + n0 + tid] = acc[r];
+    }
+}
+
+template <bool GATEUP>
+static int f32_stream_launch(MummuMoe* m, SimtArgs& a, int experts, int64_t max_rows, bool r16, cudaStream_t s,
+                             const char* name) {
+    if (max_rows <= 0) return MUMMU_OK;
+    const int R = r16 ? 16 : 8;
+    const dim3 grid((a.N + (GATEUP ? 63 : 127)) / (GATEUP ? 64 : 128), (unsigned)((max_rows + R - 1) / R), experts);
+    LaunchScope scope(m, s, name);
+    if (r16) {
+        MUMMU_CUDA_TRY(allow_big_smem(f32_stream_kernel<16, GATEUP>, m->cfg.device));
+        f32_stream_kernel<16, GATEUP><<<grid, FS_ROWS, fs_smem_bytes<16>(), s>>>(a);
+    } else {
+        MUMMU_CUDA_TRY(allow_big_smem(f32_stream_kernel<8, GATEUP>, m->cfg.device));
+        f32_stream_kernel<8, GATEUP><<<grid, FS_ROWS, fs_smem_bytes<8>(), s>>>(a);
+    }
+    MUMMU_CUDA_TRY(cudaGetLastError());
+    return MUMMU_OK;
+}
+
 template <typename TA, typename TW, bool GATEUP, typename TO>
 static int simt_launch(MummuMoe* m, SimtArgs& a, int experts, int64_t max_rows, cudaStream_t s,
                        const char* name) {
@@ -1692,7 +1818,7 @@ static int simt_launch(MummuMoe* m, SimtArgs& a, int experts, int64_t max_rows, 
 template <typename TA, typename TW>
 static int simt_two_stage(MummuMoe* m, const void* x, const int32_t* row_index,
                           const int32_t* counts, const int32_t* offsets, int64_t max_rows,
-                          void* ys, int ys_dtype, int expert_only, int rows_single, cudaStream_t s) {
+                          int64_t total_rows, void* ys, int ys_dtype, int expert_only, int rows_single, cudaStream_t s) {
     const MummuMoeConfig& c = m->cfg;
     SimtArgs a{};
     a.A = x;
@@ -1711,7 +1837,14 @@ static int simt_two_stage(MummuMoe* m, const void* x, const int32_t* row_index,
     a.N = c.inter;
     a.K = c.hidden;
     int experts = expert_only >= 0 ? 1 : c.experts_local;
-    int rc = simt_launch<TA, TW, true, float>(m, a, experts, max_rows, s, "simt_gate_up");
+    // Up to 16 rows per expert on average f32 weights stream; beyond, the tile kernel's reuse wins.  Rows of
+    // 16-byte pieces only (the copies are that wide).
+    const bool stream = std::is_same<TA, float>::value && std::is_same<TW, float>::value && ys_dtype == MUMMU_F32 &&
+                        total_rows <= 16 * (int64_t)experts && c.hidden % 4 == 0 && c.inter % 4 == 0 &&
+                        (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    const bool r16 = total_rows > 4 * (int64_t)experts;
+    int rc = stream ? f32_stream_launch<true>(m, a, experts, max_rows, r16, s, "simt_gate_up")
+                    : simt_launch<TA, TW, true, float>(m, a, experts, max_rows, s, "simt_gate_up");
     if (rc) return rc;
     SimtArgs d{};
     d.A = m->hact;
@@ -1729,6 +1862,7 @@ static int simt_two_stage(MummuMoe* m, const void* x, const int32_t* row_index,
     d.ldo = c.hidden;
     d.N = c.hidden;
     d.K = c.inter;
+    if (stream) return f32_stream_launch<false>(m, d, experts, max_rows, r16, s, "simt_down");
     switch (ys_dtype) {
         case MUMMU_F32: return simt_launch<float, TW, false, float>(m, d, experts, max_rows, s, "simt_down");
         case MUMMU_F16: return simt_launch<float, TW, false, __half>(m, d, experts, max_rows, s, "simt_down");
@@ -1740,16 +1874,16 @@ static int simt_two_stage(MummuMoe* m, const void* x, const int32_t* row_index,
 
 template <typename TA>
 static int simt_by_weight(MummuMoe* m, const void* x, const int32_t* row_index,
-                          const int32_t* counts, const int32_t* offsets, int64_t max_rows, void* ys,
-                          int ys_dtype, int expert_only, int rows_single, cudaStream_t s) {
+                          const int32_t* counts, const int32_t* offsets, int64_t max_rows,
+                          int64_t total_rows, void* ys, int ys_dtype, int expert_only, int rows_single, cudaStream_t s) {
     switch (m->cfg.weight_dtype) {
-        case MUMMU_F32: return simt_two_stage<TA, float>(m, x, row_index, counts, offsets, max_rows, ys, ys_dtype, expert_only, rows_single, s);
-        case MUMMU_F16: return simt_two_stage<TA, __half>(m, x, row_index, counts, offsets, max_rows, ys, ys_dtype, expert_only, rows_single, s);
-        case MUMMU_BF16: return simt_two_stage<TA, __nv_bfloat16>(m, x, row_index, counts, offsets, max_rows, ys, ys_dtype, expert_only, rows_single, s);
-        case MUMMU_Q4_K: return simt_two_stage<TA, q4k_t>(m, x, row_index, counts, offsets, max_rows, ys, ys_dtype, expert_only, rows_single, s);
-        case MUMMU_Q8_0: return simt_two_stage<TA, q80_t>(m, x, row_index, counts, offsets, max_rows, ys, ys_dtype, expert_only, rows_single, s);
-        case MUMMU_Q5_K: return simt_two_stage<TA, q5k_t>(m, x, row_index, counts, offsets, max_rows, ys, ys_dtype, expert_only, rows_single, s);
-        case MUMMU_Q6_K: return simt_two_stage<TA, q6k_t>(m, x, row_index, counts, offsets, max_rows, ys, ys_dtype, expert_only, rows_single, s);
+        case MUMMU_F32: return simt_two_stage<TA, float>(m, x, row_index, counts, offsets, max_rows, total_rows, ys, ys_dtype, expert_only, rows_single, s);
+        case MUMMU_F16: return simt_two_stage<TA, __half>(m, x, row_index, counts, offsets, max_rows, total_rows, ys, ys_dtype, expert_only, rows_single, s);
+        case MUMMU_BF16: return simt_two_stage<TA, __nv_bfloat16>(m, x, row_index, counts, offsets, max_rows, total_rows, ys, ys_dtype, expert_only, rows_single, s);
+        case MUMMU_Q4_K: return simt_two_stage<TA, q4k_t>(m, x, row_index, counts, offsets, max_rows, total_rows, ys, ys_dtype, expert_only, rows_single, s);
+        case MUMMU_Q8_0: return simt_two_stage<TA, q80_t>(m, x, row_index, counts, offsets, max_rows, total_rows, ys, ys_dtype, expert_only, rows_single, s);
+        case MUMMU_Q5_K: return simt_two_stage<TA, q5k_t>(m, x, row_index, counts, offsets, max_rows, total_rows, ys, ys_dtype, expert_only, rows_single, s);
+        case MUMMU_Q6_K: return simt_two_stage<TA, q6k_t>(m, x, row_index, counts, offsets, max_rows, total_rows, ys, ys_dtype, expert_only, rows_single, s);
     }
     set_error("experts: bad weight dtype %d", m->cfg.weight_dtype);
     return MUMMU_ERR_CONTRACT;
@@ -1761,9 +1895,9 @@ int launch_experts_simt(MummuMoe* m, const void* x, int x_dtype, const int32_t* 
                         cudaStream_t s) {
     int rows_single = expert_only >= 0 ? (int)total_rows : 0;
     switch (x_dtype) {
-        case MUMMU_F32: return simt_by_weight<float>(m, x, row_index, counts, offsets, max_rows_per_expert, ys, ys_dtype, expert_only, rows_single, s);
-        case MUMMU_F16: return simt_by_weight<__half>(m, x, row_index, counts, offsets, max_rows_per_expert, ys, ys_dtype, expert_only, rows_single, s);
-        case MUMMU_BF16: return simt_by_weight<__nv_bfloat16>(m, x, row_index, counts, offsets, max_rows_per_expert, ys, ys_dtype, expert_only, rows_single, s);
+        case MUMMU_F32: return simt_by_weight<float>(m, x, row_index, counts, offsets, max_rows_per_expert, total_rows, ys, ys_dtype, expert_only, rows_single, s);
+        case MUMMU_F16: return simt_by_weight<__half>(m, x, row_index, counts, offsets, max_rows_per_expert, total_rows, ys, ys_dtype, expert_only, rows_single, s);
+        case MUMMU_BF16: return simt_by_weight<__nv_bfloat16>(m, x, row_index, counts, offsets, max_rows_per_expert, total_rows, ys, ys_dtype, expert_only, rows_single, s);
     }
     set_error("experts: bad activation dtype %d", x_dtype);
     return MUMMU_ERR_CONTRACT;
