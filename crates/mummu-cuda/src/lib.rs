@@ -155,6 +155,12 @@ pub mod sys {
         pub fn mummu_trunk_kv_write(trunk: *mut MummuTrunk, layer: i32, slot: i32, first: i32, count: i32, k: *const c_void,
                                     v: *const c_void, stream: *mut c_void) -> i32;
         pub fn mummu_trunk_static_bytes(cfg: *const MummuTrunkConfig) -> u64;
+        pub fn mummu_rows_add_rms(x: *mut c_void, y: *const c_void, gamma: *const f32, h: *mut c_void, rows: i64, width: i32,
+                                  eps: f32, device: i32, stream: *mut c_void) -> i32;
+        pub fn mummu_rows_qkv(q: *const c_void, k: *const c_void, v: *const c_void, gamma_q: *const f32, gamma_k: *const f32,
+                              cos: *const f32, sin: *const f32, q_out: *mut c_void, k_cache: *mut c_void,
+                              v_cache: *mut c_void, batch: i32, len: i32, past: i32, heads: i32, kv_heads: i32,
+                              head_dim: i32, max_ctx: i32, eps: f32, device: i32, stream: *mut c_void) -> i32;
         // diagnostics
         pub fn mummu_cuda_last_error() -> *const c_char;
         pub fn mummu_cuda_version() -> *const c_char;

@@ -434,6 +434,19 @@ int32_t mummu_trunk_head(MummuTrunk* trunk, void* x, const void* y_prev, int32_t
 int32_t mummu_trunk_kv_write(MummuTrunk* trunk, int32_t layer, int32_t slot, int32_t first,
                              int32_t count, const void* k, const void* v, void* stream);
 
+/* Prompt rows (many positions at once), f16 on the device, rows on 16-byte boundaries.
+ * x (+= y, may be NULL); h = rmsnorm(x) * gamma: [rows, width] (models/olmoe.rs:561-566). */
+int32_t mummu_rows_add_rms(void* x, const void* y, const float* gamma, void* h, int64_t rows, int32_t width,
+                           float eps, int32_t device, void* stream);
+/* Projections of `len` positions from `past` of each of `batch` sequences: RMSNorm of q and of k over
+ * the whole projection, rotate-half RoPE (cos, sin: f32 [max_ctx, head_dim]); q_out laid out as q (and may
+ * be q), k and v into the caches [batch, kv_heads, max_ctx, head_dim] (nn/attention.rs:196-200,
+ * nn/rope.rs:66-105). */
+int32_t mummu_rows_qkv(const void* q, const void* k, const void* v, const float* gamma_q, const float* gamma_k,
+                       const float* cos, const float* sin, void* q_out, void* k_cache, void* v_cache,
+                       int32_t batch, int32_t len, int32_t past, int32_t heads, int32_t kv_heads,
+                       int32_t head_dim, int32_t max_ctx, float eps, int32_t device, void* stream);
+
 const char* mummu_cuda_last_error(void);
 const char* mummu_cuda_version(void);
 

@@ -110,6 +110,9 @@ SYMBOLS = {
                                      C.c_void_p]),
     "mummu_trunk_kv_write": (C.c_int32, [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_void_p,
                                          C.c_void_p, C.c_void_p]),
+    "mummu_rows_add_rms": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_float,
+                                       C.c_int32, C.c_void_p]),
+    "mummu_rows_qkv": (C.c_int32, [C.c_void_p] * 10 + [C.c_int32] * 7 + [C.c_float, C.c_int32, C.c_void_p]),
     "mummu_cuda_last_error": (C.c_char_p, []),
     "mummu_cuda_version": (C.c_char_p, []),
 }

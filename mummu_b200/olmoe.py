@@ -204,15 +204,22 @@ class OlmoeDecoder:
         B, t = ids.shape
         nh, nkv, hd, H = c.num_attention_heads, c.num_key_value_heads, c.head_dim, c.hidden_size
         x = self.embed[ids]                                                         # [B, t, H]
+        y = None                                             # the last layer's expert output, not yet in x
         cos, sin = self.cos[past:past + t], self.sin[past:past + t]
+        fused = x.numel() > 0 and x.dtype == self.dtype and B <= self.max_batch and past + t <= self.max_ctx \
+            and self._rows_supported()
         for l, lay in enumerate(self.layers):
-            h = self._rms(x, lay["in_norm"])
-            q = self._rms(F.linear(h, lay["q"]), lay["q_norm"]).view(B, t, nh, hd).transpose(1, 2)
-            k = self._rms(F.linear(h, lay["k"]), lay["k_norm"]).view(B, t, nkv, hd).transpose(1, 2)
-            v = F.linear(h, lay["v"]).view(B, t, nkv, hd).transpose(1, 2)
-            q, k = self._rope(q, cos, sin), self._rope(k, cos, sin)
-            self.k_cache[l, :B, :, past:past + t] = k
-            self.v_cache[l, :B, :, past:past + t] = v
+            if fused:
+                h = self._rows_add_rms(x, y, lay["in_norm"])
+                q = self._rows_qkv(l, lay, h, past)
+            else:
+                h = self._rms(x, lay["in_norm"])
+                q = self._rms(F.linear(h, lay["q"]), lay["q_norm"]).view(B, t, nh, hd).transpose(1, 2)
+                k = self._rms(F.linear(h, lay["k"]), lay["k_norm"]).view(B, t, nkv, hd).transpose(1, 2)
+                v = F.linear(h, lay["v"]).view(B, t, nkv, hd).transpose(1, 2)
+                q, k = self._rope(q, cos, sin), self._rope(k, cos, sin)
+                self.k_cache[l, :B, :, past:past + t] = k
+                self.v_cache[l, :B, :, past:past + t] = v
             keys, vals = self.k_cache[l, :B, :, :past + t], self.v_cache[l, :B, :, :past + t]
             if nkv != nh:
                 keys = keys.repeat_interleave(nh // nkv, 1)
@@ -225,11 +232,51 @@ class OlmoeDecoder:
                     ctx = F.scaled_dot_product_attention(q, keys, vals, is_causal=(t > 1 and past == 0))
             else:
                 ctx = self._attn_masked(q, keys, vals, past)
-            x = x + F.linear(ctx.transpose(1, 2).reshape(B, t, H), lay["o"])
-            h2 = self._rms(x, lay["post_norm"])
-            x = x + lay["mlp"].forward(h2.reshape(B * t, H), c.num_experts_per_tok, c.norm_topk_prob).view(B, t, H)
-        x = self._rms(x[:, -1], self.final_norm)
+            o = F.linear(ctx.transpose(1, 2).reshape(B, t, H), lay["o"])
+            if fused:
+                h2 = self._rows_add_rms(x, o, lay["post_norm"])
+            else:
+                x = x + o
+                h2 = self._rms(x, lay["post_norm"])
+            y = lay["mlp"].forward(h2.reshape(B * t, H), c.num_experts_per_tok, c.norm_topk_prob).view(B, t, H)
+            if not fused:
+                x = x + y
+        x = x[:, -1]
+        if fused and y is not None:
+            x = x + y[:, -1]
+        x = self._rms(x, self.final_norm)
         return F.linear(x, self.lm_head).float()
+
+    # ---- prompt rows: normalisation, RoPE and cache writes in one pass each (trunk.cu) ------------
+    def _rows_supported(self) -> bool:
+        """Row widths the row kernels take: 16-byte pieces, half a head a whole number of them."""
+        c = self.cfg
+        return (c.hidden_size % 8 == 0 and c.hidden_size <= 8192 and c.head_dim % 16 == 0
+                and c.num_attention_heads * c.head_dim <= 8192 and self.k_cache.is_contiguous())
+
+    def _gamma(self, g):
+        return g if g.dtype == self.torch.float32 and g.is_contiguous() else g.float().contiguous()
+
+    def _rows_add_rms(self, x, y, gamma):
+        h, gamma = self.torch.empty_like(x), self._gamma(gamma)
+        rows, width = x.numel() // x.shape[-1], x.shape[-1]
+        moe_mod._check(L.lib.mummu_rows_add_rms(x.data_ptr(), None if y is None else y.data_ptr(), gamma.data_ptr(),
+                                                h.data_ptr(), rows, width, self.cfg.rms_norm_eps, self.dev.index,
+                                                moe_mod._torch_stream()))
+        return h
+
+    def _rows_qkv(self, l, lay, h, past):
+        t_, c = self.torch, self.cfg
+        F = t_.nn.functional
+        B, t = h.shape[:2]
+        q, k, v = F.linear(h, lay["q"]), F.linear(h, lay["k"]), F.linear(h, lay["v"])
+        gq, gk = self._gamma(lay["q_norm"]), self._gamma(lay["k_norm"])
+        moe_mod._check(L.lib.mummu_rows_qkv(q.data_ptr(), k.data_ptr(), v.data_ptr(), gq.data_ptr(), gk.data_ptr(),
+                                            self.cos.data_ptr(), self.sin.data_ptr(), q.data_ptr(),
+                                            self.k_cache[l].data_ptr(), self.v_cache[l].data_ptr(), B, t, past,
+                                            c.num_attention_heads, c.num_key_value_heads, c.head_dim, self.max_ctx,
+                                            c.rms_norm_eps, self.dev.index, moe_mod._torch_stream()))
+        return q.view(B, t, c.num_attention_heads, c.head_dim).transpose(1, 2)
 
     def _attn_masked(self, q, keys, vals, past):
         t_ = self.torch
