@@ -258,7 +258,7 @@ static int forward_device(MummuMoe* m, const void* x, void* y, int64_t tokens, i
         if (m->sw.checked && (rc = launch_check_plan(m, m->ids, m->pos, m->row_token, m->counts, m->offsets, tokens, top_k, s)))
             return rc;
         if ((rc = launch_gather_rows(m, x, m->row_token, m->xs, tokens * top_k, s))) return rc;
-        if ((rc = launch_experts_tc(m, m->xs, m->cap_tokens * c.top_k, m->counts, m->offsets, m->ys, c.act_dtype, s)))
+        if ((rc = launch_experts_tc(m, m->xs, m->cap_tokens * c.top_k, tokens * top_k, m->counts, m->offsets, m->ys, c.act_dtype, s)))
             return rc;
         return launch_combine(m, m->ys, c.act_dtype, m->ids, m->wts, m->pos, tokens, top_k, y, s);
     } else if (q4k_tc_supported(c, tokens * top_k) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && !m->sw.no_tc) {
@@ -268,7 +268,7 @@ static int forward_device(MummuMoe* m, const void* x, void* y, int64_t tokens, i
         if (m->sw.checked && (rc = launch_check_plan(m, m->ids, m->pos, m->row_token, m->counts, m->offsets, tokens, top_k, s)))
             return rc;
         if ((rc = launch_gather_rows(m, x, m->row_token, m->xs, tokens * top_k, s))) return rc;
-        if ((rc = launch_experts_q4k_tc(m, m->xs, m->cap_tokens * c.top_k, m->counts, m->offsets, m->ys, c.act_dtype, s)))
+        if ((rc = launch_experts_q4k_tc(m, m->xs, m->cap_tokens * c.top_k, tokens * top_k, m->counts, m->offsets, m->ys, c.act_dtype, s)))
             return rc;
         return launch_combine(m, m->ys, c.act_dtype, m->ids, m->wts, m->pos, tokens, top_k, y, s);
     } else {
@@ -604,7 +604,7 @@ static int32_t experts_rows(MummuMoe* m, const void* xs, const int32_t* counts, 
     }
     if (!planned && (rc = launch_offsets_from_counts(m, counts, m->cfg.experts_local, m->offsets, s))) return rc;
     if (prefill_tc_supported(m->cfg, rows) && (reinterpret_cast<uintptr_t>(xs) & 15) == 0 && !m->sw.no_tc)
-        return launch_experts_tc(m, xs, rows, counts, m->offsets, ys, m->cfg.act_dtype, s);
+        return launch_experts_tc(m, xs, rows, rows, counts, m->offsets, ys, m->cfg.act_dtype, s);
     // A shard with few experts and many rows each (expert parallelism over many ranks at decode
     // sizes: 8 experts x 64 rows): the packed-weight kernels would expand every expert's weights once
     // per 16-row pass; expanding them once to f16 and running the tensor-core GEMMs is cheaper.
@@ -613,7 +613,7 @@ static int32_t experts_rows(MummuMoe* m, const void* xs, const int32_t* counts, 
     const int64_t rows_per_expert = (int64_t)rows / shards / m->cfg.experts_local;
     const bool few_fat_experts = m->cfg.experts_local <= 8 && rows_per_expert >= 32;
     if (few_fat_experts && q4k_tc_supported(m->cfg, rows) && (reinterpret_cast<uintptr_t>(xs) & 15) == 0 && !m->sw.no_tc)
-        return launch_experts_q4k_tc(m, xs, rows, counts, m->offsets, ys, m->cfg.act_dtype, s);
+        return launch_experts_q4k_tc(m, xs, rows, rows, counts, m->offsets, ys, m->cfg.act_dtype, s);
     if (m->cfg.weight_dtype == MUMMU_Q4_K && m->cfg.act_dtype == MUMMU_F16 && (reinterpret_cast<uintptr_t>(xs) & 15) == 0 &&
         rows <= 8192 && m->cfg.hidden <= 8192 && m->cfg.inter <= 8192) {
         // decode regime: packed-weight kernels (f32 out), then narrowed to the activation dtype
@@ -621,7 +621,7 @@ static int32_t experts_rows(MummuMoe* m, const void* xs, const int32_t* counts, 
         return launch_narrow((const float*)m->ys, ys, m->cfg.act_dtype, (int64_t)rows * m->cfg.hidden, s);
     }
     if (q4k_tc_supported(m->cfg, rows) && (reinterpret_cast<uintptr_t>(xs) & 15) == 0 && !m->sw.no_tc)
-        return launch_experts_q4k_tc(m, xs, rows, counts, m->offsets, ys, m->cfg.act_dtype, s);
+        return launch_experts_q4k_tc(m, xs, rows, rows, counts, m->offsets, ys, m->cfg.act_dtype, s);
     return launch_experts_simt(m, xs, m->cfg.act_dtype, nullptr, counts, m->offsets, rows, rows, ys,
                                m->cfg.act_dtype, -1, s);
 }
@@ -674,7 +674,7 @@ static int expert_rows_device(MummuMoe* m, int expert, const void* xs, int rows,
     int rc;
     if ((rc = launch_single_expert_plan(m, expert, rows, s))) return rc;
     if (prefill_tc_supported(c, rows) && (reinterpret_cast<uintptr_t>(xs) & 15) == 0 && !m->sw.no_tc)
-        return launch_experts_tc(m, xs, rows, m->counts, m->offsets, ys, c.act_dtype, s);
+        return launch_experts_tc(m, xs, rows, rows, m->counts, m->offsets, ys, c.act_dtype, s);
     if (c.weight_dtype == MUMMU_Q4_K && c.act_dtype == MUMMU_F16 && (reinterpret_cast<uintptr_t>(xs) & 15) == 0 &&
         rows <= 8192 && c.hidden <= 8192 && c.inter <= 8192) {
         if ((rc = launch_decode_q4k_rows(m, xs, nullptr, m->counts, m->offsets, rows, (float*)m->ys, s))) return rc;

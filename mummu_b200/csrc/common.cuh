@@ -317,9 +317,9 @@ int launch_gather_rows(MummuMoe* m, const void* x, const int32_t* row_token, voi
                        cudaStream_t s);
 int launch_block_expand_f16(MummuMoe* m, int which, __half* dst, const int32_t* counts, cudaStream_t s);
 bool q4k_tc_supported(const MummuMoeConfig& c, int64_t rows_total);
-int launch_experts_q4k_tc(MummuMoe* m, const void* xs, int64_t rows_cap, const int32_t* counts, const int32_t* offsets,
+int launch_experts_q4k_tc(MummuMoe* m, const void* xs, int64_t rows_cap, int64_t rows_est, const int32_t* counts, const int32_t* offsets,
                           void* ys, int ys_dtype, cudaStream_t s);
-int launch_experts_tc(MummuMoe* m, const void* xs, int64_t rows_cap, const int32_t* counts,
+int launch_experts_tc(MummuMoe* m, const void* xs, int64_t rows_cap, int64_t rows_est, const int32_t* counts,
                       const int32_t* offsets, void* ys, int ys_dtype, cudaStream_t s);
 
 // ---- decode_q4k.cu ----

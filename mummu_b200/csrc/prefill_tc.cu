@@ -82,9 +82,113 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, fl
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
+// One warp's quarter of a finished 128 x 256 accumulator (t0: its TMEM address) to where its rows go.
+template <typename TIN, typename TOUT, bool FUSED>
+__device__ __forceinline__ void tile_epilogue(const TcArgs& a, uint32_t t0, int row0, int row_end, int nt, uint32_t quarter,
+                                              int lane, unsigned char* epi_stage) {
+                const int row = row0 + (int)quarter * 32 + lane;
+                const bool valid = row < row_end;
+                            if constexpr (FUSED) {
+                    TOUT* orow = reinterpret_cast<TOUT*>(a.out) + (size_t)row * a.ld_out + (size_t)nt * 128;
+    #pragma unroll 1
+                    for (int c = 0; c < 128; c += 32) {
+                        uint32_t g[32], u[32];
+                        tmem_ld32(t0 + c, g);
+                        tmem_ld32(t0 + 128 + c, u);
+                        tmem_ld_wait();
+                        if (valid) {
+    #pragma unroll
+                            for (int j = 0; j < 32; j += 8) {
+                                uint4 v;
+                                v.x = pack2<TOUT>(silu_fast(__uint_as_float(g[j + 0])) * __uint_as_float(u[j + 0]),
+                                                  silu_fast(__uint_as_float(g[j + 1])) * __uint_as_float(u[j + 1]));
+                                v.y = pack2<TOUT>(silu_fast(__uint_as_float(g[j + 2])) * __uint_as_float(u[j + 2]),
+                                                  silu_fast(__uint_as_float(g[j + 3])) * __uint_as_float(u[j + 3]));
+                                v.z = pack2<TOUT>(silu_fast(__uint_as_float(g[j + 4])) * __uint_as_float(u[j + 4]),
+                                                  silu_fast(__uint_as_float(g[j + 5])) * __uint_as_float(u[j + 5]));
+                                v.w = pack2<TOUT>(silu_fast(__uint_as_float(g[j + 6])) * __uint_as_float(u[j + 6]),
+                                                  silu_fast(__uint_as_float(g[j + 7])) * __uint_as_float(u[j + 7]));
+                                *reinterpret_cast<uint4*>(orow + c + j) = v;
+                            }
+                        }
+                    }
+                } else if constexpr (sizeof(TOUT) == 4) {
+                    TOUT* orow = reinterpret_cast<TOUT*>(a.out) + (size_t)row * a.ld_out + (size_t)nt * 256;
+    #pragma unroll 1
+                    for (int c = 0; c < 256; c += 32) {
+                        uint32_t d[32];
+                        tmem_ld32(t0 + c, d);
+                        tmem_ld_wait();
+                        if (valid) {
+    #pragma unroll
+                            for (int j = 0; j < 32; j += 4)
+                                *reinterpret_cast<uint4*>(reinterpret_cast<float*>(orow) + c + j) =
+                                    make_uint4(d[j], d[j + 1], d[j + 2], d[j + 3]);
+                        }
+                    }
+                } else {
+                    // 16-bit output: where this lane's row goes (its own buffer, or the buffer of the
+                    // rank the row came from); then 64 columns at a time through shared memory, so that
+                    // a store instruction of the warp writes 128 contiguous bytes of each of 4 rows
+                    // instead of 16 bytes of each of 32 rows - what a store across NVLink needs
+                    unsigned char* dptr = nullptr;
+                    if (valid) {
+                        if (a.ret_seg) {
+                            int lo = 0, hi = a.n_seg;                // last segment that starts at or before row
+                            while (hi - lo > 1) {
+                                const int mid = (lo + hi) >> 1;
+                                if (a.ret_seg[mid] <= row) lo = mid; else hi = mid;
+                            }
+                            const int64_t drow = (int64_t)a.ret_dst[lo] + (row - a.ret_seg[lo]);
+                            if (drow >= 0 && drow < a.back_rows)
+                                dptr = reinterpret_cast<unsigned char*>(a.back[lo % a.world]) + (size_t)drow * a.ld_out * 2;
+                            else
+                                atomicOr(a.status, STATUS_BOUNDS);
+                        } else {
+                            dptr = reinterpret_cast<unsigned char*>(a.out) + (size_t)row * a.ld_out * 2;
+                        }
+                        if (dptr) dptr += (size_t)nt * 256 * 2;
+                    }
+                    uint4* stg = reinterpret_cast<uint4*>(epi_stage + quarter * TC_EPI_STAGE_BYTES);
+    #pragma unroll 1
+                    for (int c = 0; c < 256; c += 64) {
+                        uint32_t d0[32], d1[32];
+                        tmem_ld32(t0 + c, d0);
+                        tmem_ld32(t0 + c + 32, d1);
+                        tmem_ld_wait();
+    #pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            uint4 v, w;
+                            v.x = pack2<TIN>(__uint_as_float(d0[8 * j + 0]), __uint_as_float(d0[8 * j + 1]));
+                            v.y = pack2<TIN>(__uint_as_float(d0[8 * j + 2]), __uint_as_float(d0[8 * j + 3]));
+                            v.z = pack2<TIN>(__uint_as_float(d0[8 * j + 4]), __uint_as_float(d0[8 * j + 5]));
+                            v.w = pack2<TIN>(__uint_as_float(d0[8 * j + 6]), __uint_as_float(d0[8 * j + 7]));
+                            w.x = pack2<TIN>(__uint_as_float(d1[8 * j + 0]), __uint_as_float(d1[8 * j + 1]));
+                            w.y = pack2<TIN>(__uint_as_float(d1[8 * j + 2]), __uint_as_float(d1[8 * j + 3]));
+                            w.z = pack2<TIN>(__uint_as_float(d1[8 * j + 4]), __uint_as_float(d1[8 * j + 5]));
+                            w.w = pack2<TIN>(__uint_as_float(d1[8 * j + 6]), __uint_as_float(d1[8 * j + 7]));
+                            // piece index swizzled by the row: the 32 lanes of a store hit 32 banks x 4
+                            stg[lane * 8 + (j ^ (lane & 7))] = v;
+                            stg[lane * 8 + ((j + 4) ^ (lane & 7))] = w;
+                        }
+                        __syncwarp();
+    #pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int idx = i * 32 + lane, r = idx >> 3, pc = idx & 7;
+                            const uint4 v = stg[r * 8 + (pc ^ (r & 7))];
+                            unsigned char* p = reinterpret_cast<unsigned char*>(
+                                __shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(dptr), r));
+                            if (p) *reinterpret_cast<uint4*>(p + c * 2 + pc * 16) = v;
+                        }
+                        __syncwarp();
+                    }
+                }
+}
+
 // ------------------------------------------------------------------------------------------------
 // tile list
 // ------------------------------------------------------------------------------------------------
+template <int BM>
 struct TileCursor {
     int e = 0;
     // tile index -> (expert, first sorted row, rows end of the expert, n tile)
@@ -93,11 +197,11 @@ struct TileCursor {
         while (tile >= tile_start[e + 1]) ++e;
         const int local = tile - tile_start[e];
         const int cnt = counts[e];
-        const int m_tiles = (cnt + TC_BM - 1) / TC_BM;
+        const int m_tiles = (cnt + BM - 1) / BM;
         nt = local / m_tiles;
         const int mt = local - nt * m_tiles;
         expert = e;
-        row0 = offsets[e] + mt * TC_BM;
+        row0 = offsets[e] + mt * BM;
         row_end = offsets[e] + cnt;
     }
 };
@@ -161,7 +265,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
-            TileCursor cur;
+            TileCursor<TC_BM> cur;
             uint32_t it = 0;
             bool ok = true;
             for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
@@ -226,7 +330,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     } else {
         // ---------------- epilogue: warps 2..5, TMEM lane quarter = warp % 4 ----------------
         const uint32_t quarter = warp & 3u;
-        TileCursor cur;
+        TileCursor<TC_BM> cur;
         uint32_t tcount = 0;
         bool ok = true;
         for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++tcount) {
@@ -235,104 +339,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             const uint32_t as = tcount & 1u, aph = (tcount >> 1) & 1u;
             if (!mbar_wait(tfull0 + 8 * as, aph, abort_flag)) { ok = false; break; }
             tc_fence_after();
-            const int row = row0 + (int)quarter * 32 + lane;
-            const bool valid = row < row_end;
-            const uint32_t t0 = tmem_base + ((quarter * 32u) << 16) + as * 256u;
-            if constexpr (FUSED) {
-                TOUT* orow = reinterpret_cast<TOUT*>(a.out) + (size_t)row * a.ld_out + (size_t)nt * 128;
-#pragma unroll 1
-                for (int c = 0; c < 128; c += 32) {
-                    uint32_t g[32], u[32];
-                    tmem_ld32(t0 + c, g);
-                    tmem_ld32(t0 + 128 + c, u);
-                    tmem_ld_wait();
-                    if (valid) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 8) {
-                            uint4 v;
-                            v.x = pack2<TOUT>(silu_fast(__uint_as_float(g[j + 0])) * __uint_as_float(u[j + 0]),
-                                              silu_fast(__uint_as_float(g[j + 1])) * __uint_as_float(u[j + 1]));
-                            v.y = pack2<TOUT>(silu_fast(__uint_as_float(g[j + 2])) * __uint_as_float(u[j + 2]),
-                                              silu_fast(__uint_as_float(g[j + 3])) * __uint_as_float(u[j + 3]));
-                            v.z = pack2<TOUT>(silu_fast(__uint_as_float(g[j + 4])) * __uint_as_float(u[j + 4]),
-                                              silu_fast(__uint_as_float(g[j + 5])) * __uint_as_float(u[j + 5]));
-                            v.w = pack2<TOUT>(silu_fast(__uint_as_float(g[j + 6])) * __uint_as_float(u[j + 6]),
-                                              silu_fast(__uint_as_float(g[j + 7])) * __uint_as_float(u[j + 7]));
-                            *reinterpret_cast<uint4*>(orow + c + j) = v;
-                        }
-                    }
-                }
-            } else if constexpr (sizeof(TOUT) == 4) {
-                TOUT* orow = reinterpret_cast<TOUT*>(a.out) + (size_t)row * a.ld_out + (size_t)nt * 256;
-#pragma unroll 1
-                for (int c = 0; c < 256; c += 32) {
-                    uint32_t d[32];
-                    tmem_ld32(t0 + c, d);
-                    tmem_ld_wait();
-                    if (valid) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4)
-                            *reinterpret_cast<uint4*>(reinterpret_cast<float*>(orow) + c + j) =
-                                make_uint4(d[j], d[j + 1], d[j + 2], d[j + 3]);
-                    }
-                }
-            } else {
-                // 16-bit output: where this lane's row goes (its own buffer, or the buffer of the
-                // rank the row came from); then 64 columns at a time through shared memory, so that
-                // a store instruction of the warp writes 128 contiguous bytes of each of 4 rows
-                // instead of 16 bytes of each of 32 rows - what a store across NVLink needs
-                unsigned char* dptr = nullptr;
-                if (valid) {
-                    if (a.ret_seg) {
-                        int lo = 0, hi = a.n_seg;                // last segment that starts at or before row
-                        while (hi - lo > 1) {
-                            const int mid = (lo + hi) >> 1;
-                            if (a.ret_seg[mid] <= row) lo = mid; else hi = mid;
-                        }
-                        const int64_t drow = (int64_t)a.ret_dst[lo] + (row - a.ret_seg[lo]);
-                        if (drow >= 0 && drow < a.back_rows)
-                            dptr = reinterpret_cast<unsigned char*>(a.back[lo % a.world]) + (size_t)drow * a.ld_out * 2;
-                        else
-                            atomicOr(a.status, STATUS_BOUNDS);
-                    } else {
-                        dptr = reinterpret_cast<unsigned char*>(a.out) + (size_t)row * a.ld_out * 2;
-                    }
-                    if (dptr) dptr += (size_t)nt * 256 * 2;
-                }
-                uint4* stg = reinterpret_cast<uint4*>(epi_stage + quarter * TC_EPI_STAGE_BYTES);
-#pragma unroll 1
-                for (int c = 0; c < 256; c += 64) {
-                    uint32_t d0[32], d1[32];
-                    tmem_ld32(t0 + c, d0);
-                    tmem_ld32(t0 + c + 32, d1);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        uint4 v, w;
-                        v.x = pack2<TIN>(__uint_as_float(d0[8 * j + 0]), __uint_as_float(d0[8 * j + 1]));
-                        v.y = pack2<TIN>(__uint_as_float(d0[8 * j + 2]), __uint_as_float(d0[8 * j + 3]));
-                        v.z = pack2<TIN>(__uint_as_float(d0[8 * j + 4]), __uint_as_float(d0[8 * j + 5]));
-                        v.w = pack2<TIN>(__uint_as_float(d0[8 * j + 6]), __uint_as_float(d0[8 * j + 7]));
-                        w.x = pack2<TIN>(__uint_as_float(d1[8 * j + 0]), __uint_as_float(d1[8 * j + 1]));
-                        w.y = pack2<TIN>(__uint_as_float(d1[8 * j + 2]), __uint_as_float(d1[8 * j + 3]));
-                        w.z = pack2<TIN>(__uint_as_float(d1[8 * j + 4]), __uint_as_float(d1[8 * j + 5]));
-                        w.w = pack2<TIN>(__uint_as_float(d1[8 * j + 6]), __uint_as_float(d1[8 * j + 7]));
-                        // piece index swizzled by the row: the 32 lanes of a store hit 32 banks x 4
-                        stg[lane * 8 + (j ^ (lane & 7))] = v;
-                        stg[lane * 8 + ((j + 4) ^ (lane & 7))] = w;
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int idx = i * 32 + lane, r = idx >> 3, pc = idx & 7;
-                        const uint4 v = stg[r * 8 + (pc ^ (r & 7))];
-                        unsigned char* p = reinterpret_cast<unsigned char*>(
-                            __shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(dptr), r));
-                        if (p) *reinterpret_cast<uint4*>(p + c * 2 + pc * 16) = v;
-                    }
-                    __syncwarp();
-                }
-            }
+            tile_epilogue<TIN, TOUT, FUSED>(a, tmem_base + ((quarter * 32u) << 16) + as * 256u, row0, row_end, nt, quarter, lane,
+                                            epi_stage);
             tc_fence_before();
             mbar_arrive(tempty0 + 8 * as);
         }
@@ -345,6 +353,184 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         __syncwarp();
         tc_fence_after();
         tmem_dealloc(tmem_base, TC_TMEM_COLS);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// The same GEMM on pairs of CTAs (cta_group::2): a tile is 256 rows x 256 columns, each CTA of the pair
+// loads its 128 rows of A and one half of B (gate or up rows; or 128 of the 256 output columns) and keeps
+// 128 accumulator rows; the leader issues the MMAs for both.  A stage is 32 KB a CTA instead of 48, so L2
+// sends two thirds of the bytes per MMA and shared memory holds six stages instead of four.  Tiles are
+// twice as tall: experts with few rows waste more of them.  Measured (gate/up + down): 16384 tokens on 128
+// experts (1024 rows each) 654 + 388 -> 628 + 369 us; 4096 tokens, skewed, on 64 (512 rows) 247 + 140 -> 245 + 135
+// but the call 586 -> 597 us; 2048 tokens (256 rows) 2 % slower.  So pairs run from TP_MIN_ROWS rows per expert.
+// ------------------------------------------------------------------------------------------------
+constexpr int TP_BM = 256, TP_STAGES = 6, TP_MIN_ROWS = 768;
+constexpr uint32_t TP_STAGE_BYTES = 2 * TC_BM * TC_BK * 2;   // this CTA's A rows and half of B = 32 KiB
+
+template <typename TIN, typename TOUT, bool FUSED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
+grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b0,
+                         const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ TcArgs a) {
+    extern __shared__ unsigned char smem_dyn[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
+    unsigned char* tiles = smem;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + TP_STAGES * TP_STAGE_BYTES);
+    // bars: full[S] (used in the leader), empty[S], tmem_full[2], tmem_empty[2] (used in the leader), end
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * TP_STAGES + 5);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* tile_start = reinterpret_cast<int*>(tmem_slot + 2);
+    unsigned char* epi_stage = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(tile_start + a.E + 1) + 15) & ~(uintptr_t)15);
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
+    const uint32_t rank = cluster_rank();
+    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + TP_STAGES);
+    const uint32_t tfull0 = smem_u32(bars + 2 * TP_STAGES), tempty0 = smem_u32(bars + 2 * TP_STAGES + 2);
+    const uint32_t end_bar = smem_u32(bars + 2 * TP_STAGES + 4);
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+
+    if (tid == 0) {
+        *abort_flag = 0;
+        for (int s = 0; s < TP_STAGES; ++s) {
+            mbar_init(full0 + 8 * s, 1);
+            mbar_init(empty0 + 8 * s, 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(tfull0 + 8 * s, 1);
+            mbar_init(tempty0 + 8 * s, 8);           // the four epilogue warps of both CTAs
+        }
+        mbar_init(end_bar, 1);
+        mbar_init_fence();
+        fence_proxy_async_smem();
+    }
+    if (warp == 1) {
+        tmem_alloc_pair(smem_u32(tmem_slot), TC_TMEM_COLS);
+        tmem_relinquish_pair();
+    }
+    if (warp == 2) {
+        int acc = 0;
+        for (int e0 = 0; e0 < a.E; e0 += 32) {
+            const int e = e0 + lane;
+            const int c = e < a.E ? ((a.counts[e] + TP_BM - 1) / TP_BM) * a.n_tiles : 0;
+            int incl = c;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int up = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+                if (lane >= off) incl += up;
+            }
+            if (e < a.E) tile_start[e] = acc + incl - c;
+            acc += __shfl_sync(0xFFFFFFFFu, incl, 31);
+        }
+        if (lane == 0) tile_start[a.E] = acc;
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                  // both CTAs' barriers are there before anyone signals them
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const int total_tiles = tile_start[a.E];
+    const int k_blocks = a.K / TC_BK;
+
+    if (warp == 0) {
+        // ---------------- TMA producer (both CTAs) ----------------
+        if (lane == 0) {
+            TileCursor<TP_BM> cur;
+            uint32_t it = 0;
+            bool ok = true;
+            const uint32_t full_leader = map_rank(full0, 0);
+            const CUtensorMap* map_b = rank ? &map_b1 : &map_b0;
+            for (int tile = pair; ok && tile < total_tiles; tile += pairs) {
+                int e, row0, row_end, nt;
+                cur.locate(tile_start, a.counts, a.offsets, tile, a.n_tiles, e, row0, row_end, nt);
+                const int arow = row0 + (int)rank * TC_BM;
+                const int brow = e * a.b_rows_per_expert + nt * a.b_tile_rows + (rank ? a.b1_row_offset : 0);
+                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+                    const uint32_t s = it % TP_STAGES, ph = (it / TP_STAGES) & 1u;
+                    if (!mbar_wait(empty0 + 8 * s, ph ^ 1u, abort_flag)) { ok = false; break; }
+                    const uint32_t dst = smem_u32(tiles + s * TP_STAGE_BYTES);
+                    if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * TP_STAGE_BYTES);
+                    tma_load_2d_pair(dst, &map_a, kb * TC_BK, arow, full_leader + 8 * s);
+                    tma_load_2d_pair(dst + TC_BM * TC_BK * 2, map_b, kb * TC_BK, brow, full_leader + 8 * s);
+                }
+            }
+            // every stage asked for is released by a commit that both CTAs receive: wait for the last ones, so
+            // that neither copies nor arrivals are on their way when the shared memory goes (after giving up the
+            // waits end at once when the abort flag is up; the copies themselves are given time)
+            if (ok) {
+                for (uint32_t back = 1; back <= (uint32_t)TP_STAGES && back <= it; ++back) {
+                    const uint32_t j = it - back;
+                    if (!mbar_wait(empty0 + 8 * (j % TP_STAGES), (j / TP_STAGES) & 1u, abort_flag)) break;
+                }
+            } else {
+                for (uint32_t i = 0; i < (1u << 14); ++i) __nanosleep(64);
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------- MMA issuer (leader); the whole warp walks, one lane issues ----------------
+        if (rank == 0) {
+            const uint32_t fmt = std::is_same<TIN, __nv_bfloat16>::value ? 1u : 0u;
+            const uint32_t idesc = make_idesc(fmt, 256, 256);
+            const bool lead = elect_one();
+            uint32_t it = 0, tcount = 0;
+            bool ok = true;
+            for (int tile = pair; ok && tile < total_tiles; tile += pairs, ++tcount) {
+                const uint32_t as = tcount & 1u, aph = (tcount >> 1) & 1u;
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait(tempty0 + 8 * as, aph ^ 1u, abort_flag));
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t d0 = tmem_base + as * 256u;
+                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+                    const uint32_t s = it % TP_STAGES, ph = (it / TP_STAGES) & 1u;
+                    ok = __all_sync(0xFFFFFFFFu, mbar_wait(full0 + 8 * s, ph, abort_flag));
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t sa = smem_u32(tiles + s * TP_STAGE_BYTES);
+                    const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + TC_BM * TC_BK * 2);
+                    if (lead) {
+#pragma unroll
+                        for (int k = 0; k < TC_BK / 16; ++k) umma_f16_pair(d0, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        umma_commit_pair(empty0 + 8 * s);
+                        if (kb == k_blocks - 1) umma_commit_pair(tfull0 + 8 * as);
+                    }
+                    __syncwarp();
+                }
+            }
+            if (!ok && lead) {      // gave up: MMAs in flight end before their operands and the accumulators go away
+                umma_commit_pair(end_bar);
+                for (uint32_t i = 0; i < (1u << 16) && !mbar_test(end_bar, 0); ++i) __nanosleep(64);
+            }
+        }
+    } else {
+        // ---------------- epilogue: warps 2..5 of each CTA on its own 128 rows ----------------
+        const uint32_t quarter = warp & 3u;
+        const uint32_t tempty_leader = map_rank(tempty0, 0);
+        TileCursor<TP_BM> cur;
+        uint32_t tcount = 0;
+        bool ok = true;
+        for (int tile = pair; ok && tile < total_tiles; tile += pairs, ++tcount) {
+            int e, row0, row_end, nt;
+            cur.locate(tile_start, a.counts, a.offsets, tile, a.n_tiles, e, row0, row_end, nt);
+            const uint32_t as = tcount & 1u, aph = (tcount >> 1) & 1u;
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(tfull0 + 8 * as, aph, abort_flag));
+            if (!ok) break;
+            tc_fence_after();
+            tile_epilogue<TIN, TOUT, FUSED>(a, tmem_base + ((quarter * 32u) << 16) + as * 256u, row0 + (int)rank * TC_BM, row_end,
+                                            nt, quarter, lane, epi_stage);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(tempty_leader + 8 * as);
+        }
+    }
+    // ---------------- teardown ----------------
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                  // nobody leaves while the other may still signal it or read its operands
+    if (tid == 0 && *abort_flag) atomicOr(a.status, STATUS_TIMEOUT);
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, TC_TMEM_COLS);
     }
 }
 
@@ -424,6 +610,11 @@ bool prefill_tc_supported(const MummuMoeConfig& c, int64_t rows_total) {
            c.hidden % 256 == 0 && c.inter % 128 == 0 && rows_total >= 1;
 }
 
+static size_t tp_smem_bytes(int E) {
+    return 1024 + (size_t)TP_STAGES * TP_STAGE_BYTES + (2 * TP_STAGES + 5) * 8 + 16 + (size_t)(E + 1) * 4 + 64 + 16 +
+           4 * TC_EPI_STAGE_BYTES;
+}
+
 static size_t tc_smem_bytes(int E) {
     return 1024 + (size_t)TC_STAGES * TC_STAGE_BYTES + (2 * TC_STAGES + 4) * 8 + 16 + (size_t)(E + 1) * 4 + 64 + 16 +
            4 * TC_EPI_STAGE_BYTES;
@@ -432,7 +623,7 @@ static size_t tc_smem_bytes(int E) {
 // banks: gate, up, down as [experts_local, out, in] in the activation's 16-bit type (the handle's
 // own banks, or the expanded image of its Q4_K banks)
 template <typename TIN>
-static int launch_tc_typed(MummuMoe* m, const void* xs, int64_t rows_cap, const int32_t* counts,
+static int launch_tc_typed(MummuMoe* m, const void* xs, int64_t rows_cap, int64_t rows_est, const int32_t* counts,
                            const int32_t* offsets, void* ys, int ys_dtype, const void* const* banks, cudaStream_t s) {
     const MummuMoeConfig& c = m->cfg;
     CUtensorMap map_x, map_h, map_g, map_u, map_d;
@@ -458,7 +649,15 @@ static int launch_tc_typed(MummuMoe* m, const void* xs, int64_t rows_cap, const 
     g.out = m->hact;
     g.ld_out = c.inter;
     g.status = m->status;
-    {
+    // rows_est counts the rows of all ranks' experts (see the callers), so this is rows per expert
+    const bool pair = rows_est >= TP_MIN_ROWS * (int64_t)c.experts;
+    const size_t smem_pair = tp_smem_bytes(c.experts_local);
+    if (pair) {
+        MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_pair_kernel<TIN, TIN, true>, c.device));
+        LaunchScope scope(m, s, "tc_gate_up");
+        grouped_gemm_pair_kernel<TIN, TIN, true><<<sms & ~1, TC_THREADS, smem_pair, s>>>(map_x, map_g, map_u, g);
+        MUMMU_CUDA_TRY(cudaGetLastError());
+    } else {
         MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_tc_kernel<TIN, TIN, true>, c.device));
         LaunchScope scope(m, s, "tc_gate_up");
         grouped_gemm_tc_kernel<TIN, TIN, true><<<sms, TC_THREADS, smem, s>>>(map_x, map_g, map_u, g);
@@ -486,7 +685,10 @@ static int launch_tc_typed(MummuMoe* m, const void* xs, int64_t rows_cap, const 
         m->scatter.used = true;
     }
     LaunchScope scope(m, s, "tc_down");
-    if (ys_dtype == MUMMU_F32) {
+    if (pair && ys_dtype != MUMMU_F32) {
+        MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_pair_kernel<TIN, TIN, false>, c.device));
+        grouped_gemm_pair_kernel<TIN, TIN, false><<<sms & ~1, TC_THREADS, smem_pair, s>>>(map_h, map_d, map_d, d);
+    } else if (ys_dtype == MUMMU_F32) {
         MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_tc_kernel<TIN, float, false>, c.device));
         grouped_gemm_tc_kernel<TIN, float, false><<<sms, TC_THREADS, smem, s>>>(map_h, map_d, map_d, d);
     } else {
@@ -498,13 +700,13 @@ static int launch_tc_typed(MummuMoe* m, const void* xs, int64_t rows_cap, const 
 }
 
 // xs: sorted rows [rows_cap, hidden] in the activation dtype (rows_cap = allocated rows, used as
-// the tensor-map bound); ys: [rows, hidden] in ys_dtype (F32 or the activation dtype)
-int launch_experts_tc(MummuMoe* m, const void* xs, int64_t rows_cap, const int32_t* counts,
+// the tensor-map bound), rows_est: rows expected over all experts of the layer; ys: [rows, hidden] in ys_dtype (F32 or the activation dtype)
+int launch_experts_tc(MummuMoe* m, const void* xs, int64_t rows_cap, int64_t rows_est, const int32_t* counts,
                       const int32_t* offsets, void* ys, int ys_dtype, cudaStream_t s) {
     const void* banks[3] = {m->bank[0], m->bank[1], m->bank[2]};
     if (m->cfg.act_dtype == MUMMU_BF16)
-        return launch_tc_typed<__nv_bfloat16>(m, xs, rows_cap, counts, offsets, ys, ys_dtype, banks, s);
-    return launch_tc_typed<__half>(m, xs, rows_cap, counts, offsets, ys, ys_dtype, banks, s);
+        return launch_tc_typed<__nv_bfloat16>(m, xs, rows_cap, rows_est, counts, offsets, ys, ys_dtype, banks, s);
+    return launch_tc_typed<__half>(m, xs, rows_cap, rows_est, counts, offsets, ys, ys_dtype, banks, s);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -579,7 +781,7 @@ bool q4k_tc_supported(const MummuMoeConfig& c, int64_t rows_total) {
     return packed && c.act_dtype == MUMMU_F16 && c.hidden % 256 == 0 && c.inter % 256 == 0 && rows_total >= 1;
 }
 
-int launch_experts_q4k_tc(MummuMoe* m, const void* xs, int64_t rows_cap, const int32_t* counts, const int32_t* offsets,
+int launch_experts_q4k_tc(MummuMoe* m, const void* xs, int64_t rows_cap, int64_t rows_est, const int32_t* counts, const int32_t* offsets,
                           void* ys, int ys_dtype, cudaStream_t s) {
     const MummuMoeConfig& c = m->cfg;
     const int64_t per_bank = (int64_t)c.experts_local * c.inter * c.hidden;
@@ -609,7 +811,7 @@ int launch_experts_q4k_tc(MummuMoe* m, const void* xs, int64_t rows_cap, const i
         MUMMU_CUDA_TRY(cudaGetLastError());
     }
     const void* banks[3] = {owner->wexp[0], owner->wexp[1], owner->wexp[2]};
-    return launch_tc_typed<__half>(m, xs, rows_cap, counts, offsets, ys, ys_dtype, banks, s);
+    return launch_tc_typed<__half>(m, xs, rows_cap, rows_est, counts, offsets, ys, ys_dtype, banks, s);
 }
 
 int launch_gather_rows(MummuMoe* m, const void* x, const int32_t* row_token, void* xs, int64_t rows,

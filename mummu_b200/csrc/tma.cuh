@@ -76,6 +76,16 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
         : "memory");
 }
 
+// the same by one CTA of a pair: the tile lands in this CTA, the bytes count on a barrier of either CTA
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c_inner, int c_outer,
+                                                 uint32_t bar_cluster) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], "
+        "[%2];\n" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster), "r"(c_inner), "r"(c_outer)
+        : "memory");
+}
+
 // Host: encode a row-major 2-D view [outer, inner] (inner contiguous) with the given box.
 // Returns MUMMU_OK or MUMMU_ERR_DEVICE with the error text set.
 int encode_tiled_2d(CUtensorMap* map, const void* base, CUtensorMapDataType dtype, uint32_t elem_bytes,
