@@ -237,49 +237,34 @@ static int read_status(MummuMoe* m, cudaStream_t s) {
 static int forward_device(MummuMoe* m, const void* x, void* y, int64_t tokens, int top_k, int norm,
                           cudaStream_t s) {
     const MummuMoeConfig& c = m->cfg;
-    int rc;
-    if (decode_q4k_supported(c, tokens) && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-        // decode: router and grouping in one launch when the call is small enough
-        rc = launch_router(m, x, tokens, top_k, norm, m->ids, m->wts, m->counts, s, true);
-        if (rc == MUMMU_ERR_UNSUPPORTED) {
-            if ((rc = launch_router(m, x, tokens, top_k, norm, m->ids, m->wts, m->counts, s))) return rc;
-            rc = launch_permute(m, m->ids, tokens, top_k, m->counts, m->offsets, m->row_token, m->pos, s);
-        }
-        if (rc) return rc;
-        if (m->sw.checked && (rc = launch_check_plan(m, m->ids, m->pos, m->row_token, m->counts, m->offsets, tokens, top_k, s)))
-            return rc;
+    // router and grouping in one launch when the call is small enough (whatever runs the experts: the
+    // separate grouping is two memsets and a kernel more)
+    int rc = launch_router(m, x, tokens, top_k, norm, m->ids, m->wts, m->counts, s, true);
+    if (rc == MUMMU_ERR_UNSUPPORTED) {
+        if ((rc = launch_router(m, x, tokens, top_k, norm, m->ids, m->wts, m->counts, s))) return rc;
+        rc = launch_permute(m, m->ids, tokens, top_k, m->counts, m->offsets, m->row_token, m->pos, s);
+    }
+    if (rc) return rc;
+    if (m->sw.checked && (rc = launch_check_plan(m, m->ids, m->pos, m->row_token, m->counts, m->offsets, tokens, top_k, s)))
+        return rc;
+    const bool aligned = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    if (decode_q4k_supported(c, tokens) && aligned) {
         if ((rc = launch_decode_q4k(m, x, tokens, top_k, s))) return rc;
         return launch_combine(m, m->ys, MUMMU_F32, m->ids, m->wts, m->pos, tokens, top_k, y, s);
     }
-    if ((rc = launch_router(m, x, tokens, top_k, norm, m->ids, m->wts, m->counts, s))) return rc;
-    if (prefill_tc_supported(c, tokens * top_k) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && !m->sw.no_tc) {
-        // tensor-core path: sorted copy of the routed rows, two grouped GEMMs, 16-bit expert outputs
-        if ((rc = launch_permute(m, m->ids, tokens, top_k, m->counts, m->offsets, m->row_token, m->pos, s))) return rc;
-        if (m->sw.checked && (rc = launch_check_plan(m, m->ids, m->pos, m->row_token, m->counts, m->offsets, tokens, top_k, s)))
-            return rc;
+    const bool tc = prefill_tc_supported(c, tokens * top_k);
+    if (aligned && !m->sw.no_tc && (tc || q4k_tc_supported(c, tokens * top_k))) {
+        // tensor-core path: sorted copy of the routed rows, two grouped GEMMs, 16-bit expert outputs; Q4_K with more
+        // tokens than the packed-weight kernels take expands the experts that have rows to f16 first
         if ((rc = launch_gather_rows(m, x, m->row_token, m->xs, tokens * top_k, s))) return rc;
-        if ((rc = launch_experts_tc(m, m->xs, m->cap_tokens * c.top_k, tokens * top_k, m->counts, m->offsets, m->ys, c.act_dtype, s)))
-            return rc;
+        auto experts = tc ? launch_experts_tc : launch_experts_q4k_tc;
+        if ((rc = experts(m, m->xs, m->cap_tokens * c.top_k, tokens * top_k, m->counts, m->offsets, m->ys, c.act_dtype, s))) return rc;
         return launch_combine(m, m->ys, c.act_dtype, m->ids, m->wts, m->pos, tokens, top_k, y, s);
-    } else if (q4k_tc_supported(c, tokens * top_k) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && !m->sw.no_tc) {
-        // Q4_K with more tokens than the packed-weight kernels take: expand the experts that have
-        // rows to f16, then the tensor-core path
-        if ((rc = launch_permute(m, m->ids, tokens, top_k, m->counts, m->offsets, m->row_token, m->pos, s))) return rc;
-        if (m->sw.checked && (rc = launch_check_plan(m, m->ids, m->pos, m->row_token, m->counts, m->offsets, tokens, top_k, s)))
-            return rc;
-        if ((rc = launch_gather_rows(m, x, m->row_token, m->xs, tokens * top_k, s))) return rc;
-        if ((rc = launch_experts_q4k_tc(m, m->xs, m->cap_tokens * c.top_k, tokens * top_k, m->counts, m->offsets, m->ys, c.act_dtype, s)))
-            return rc;
-        return launch_combine(m, m->ys, c.act_dtype, m->ids, m->wts, m->pos, tokens, top_k, y, s);
-    } else {
-        if ((rc = launch_permute(m, m->ids, tokens, top_k, m->counts, m->offsets, m->row_token, m->pos, s))) return rc;
-        if (m->sw.checked && (rc = launch_check_plan(m, m->ids, m->pos, m->row_token, m->counts, m->offsets, tokens, top_k, s)))
-            return rc;
-        int64_t max_rows = tokens;  // an expert serves a token at most once
-        if ((rc = launch_experts_simt(m, x, c.act_dtype, m->row_token, m->counts, m->offsets, max_rows,
-                                      tokens * top_k, m->ys, MUMMU_F32, -1, s)))
-            return rc;
     }
+    // an expert serves a token at most once: `tokens` bounds the rows of an expert
+    if ((rc = launch_experts_simt(m, x, c.act_dtype, m->row_token, m->counts, m->offsets, tokens, tokens * top_k, m->ys, MUMMU_F32,
+                                  -1, s)))
+        return rc;
     return launch_combine(m, m->ys, MUMMU_F32, m->ids, m->wts, m->pos, tokens, top_k, y, s);
 }
 
