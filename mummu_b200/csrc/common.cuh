@@ -174,7 +174,7 @@ struct MummuSwitches {
     int no_tc = 0;            // MUMMU_CUDA_NO_TC: never take the tcgen05 grouped GEMM
     int no_host_graph = 0;    // MUMMU_CUDA_NO_HOST_GRAPH: host-pointer decode calls stay eager
     int router_plain = 0;     // MUMMU_CUDA_ROUTER_PLAIN: decode router without the bulk-copied slice image
-    int decode_no_pdl = 0;    // MUMMU_CUDA_DECODE_NO_PDL: no programmatic dependent launch of the down kernel
+    int decode_no_pdl = 0;    // MUMMU_CUDA_DECODE_NO_PDL: no programmatic dependent launches in the layer's chain
     int decode_nt = 0;        // MUMMU_CUDA_DECODE_NT: 1 forces one 8-token tile per pass
     int decode_stream_min = 0;// MUMMU_CUDA_DECODE_STREAM_MIN: row tiles from which the streaming variant runs
     int decode_rb_gateup = 0; // MUMMU_CUDA_DECODE_RB_GATEUP / _DOWN: row tiles per CTA (0 = planned)
@@ -275,6 +275,37 @@ struct LaunchScope {
     LaunchScope(MummuMoe* m_, cudaStream_t s_, const char* name_);
     ~LaunchScope();
 };
+
+// Programmatic dependent launch.  A kernel of the layer's chain may become resident while the one before
+// it drains; pdl_enter() is its first touch of memory: it waits until everything before it is complete and
+// visible, and from then on lets the next kernel come up.  A kernel that reads anything before pdl_enter()
+// reads only what no kernel of a call writes (weights), or what was complete when its predecessor passed
+// its own pdl_enter().  Returns at once after an ordinary launch.
+// Measured: one token through four Q4_K layers 169 -> 146 us, 47 tokens on bf16 experts 181 -> 168, one decode step
+// of one sequence 1152 -> 1094 us.  The streaming gate/up kernel is launched the ordinary way: coming up under the
+// router it cost 64 tokens 30 us of 400 (its CTAs fill the SMs the router's last blocks still need).
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+template <typename... Params, typename... Args>
+cudaError_t launch_chain(bool early, void (*kernel)(Params...), dim3 grid, unsigned block, size_t smem, cudaStream_t s,
+                         Args&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+// profiling brackets every launch with events, which would serialise the chain anyway
+inline bool chain_early(const MummuMoe* m) { return !m->sw.decode_no_pdl && !m->prof.enabled; }
 
 // ---- kernels_basic.cu ----
 // where the fused grouping of a decode-sized router call writes (null = the handle's own scratch)

@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 2) decode_q4k_kernel(DecodeArgs a)
     const uint32_t frag_base = (uint32_t)__cvta_generic_to_shared(s_frag);
     const uint32_t sxh_base = (uint32_t)__cvta_generic_to_shared(s_sxh);
 
+    pdl_enter();
     const int ai = blockIdx.x / a.ctas_per_expert;
     const int cb = blockIdx.x - ai * a.ctas_per_expert;
     if (ai >= *a.n_active) return;
@@ -289,6 +290,9 @@ decode_q4k_tma_kernel(DecodeArgs a, const __grid_constant__ CUtensorMap map0, co
     const uint32_t frag_base = smem_u32(s_frag);
     const uint32_t sxh_base = smem_u32(s_sxh);
 
+    // gate/up waits for the routing here.  down comes up while gate/up drains; the routing was complete when
+    // gate/up passed its own wait, so down may read it and request its first weights before it waits below.
+    if (GATEUP) pdl_enter();
     const int ai = blockIdx.x / a.ctas_per_expert;
     const int cb = blockIdx.x - ai * a.ctas_per_expert;
     if (ai >= *a.n_active) return;
@@ -332,16 +336,7 @@ decode_q4k_tma_kernel(DecodeArgs a, const __grid_constant__ CUtensorMap map0, co
     // request the first units before the tokens are staged
     for (int i = 0; i < r.depth; ++i)
         if (r.p_valid) ring_issue<GATEUP>(r, i, &map0, &map1, row_base, rt_first, rt_end, nsb, npasses, lane);
-    if (!a.pdl) {
-    } else if (GATEUP) {
-        // programmatic dependent launch: the down kernel's CTAs may take the SMs this grid leaves
-        // idle in its tail and request their first weights there
-        asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    } else {
-        // launched early (see above): the weights requested so far do not depend on the previous
-        // grid, the activations staged next do.  Returns at once after an ordinary launch.
-        asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    }
+    if (!GATEUP) pdl_enter();
 
     for (int pass0 = pass_first; pass0 < cnt; pass0 += pass_step) {
         const int npass = min(8 * NT, cnt - pass0);
@@ -381,8 +376,7 @@ static int bank_map(MummuMoe* m, int which, int row_bytes, int64_t rows, const C
 }
 
 template <int NT, bool GATEUP>
-static int launch_one(MummuMoe* m, DecodeArgs& a, int n_experts_max, bool stream, cudaStream_t s,
-                      const char* name, bool pdl = false, bool* used_tma = nullptr) {
+static int launch_one(MummuMoe* m, DecodeArgs& a, int n_experts_max, bool stream, cudaStream_t s, const char* name) {
     const int nsb = a.K >> 8;
     if (stream) {
         // deepest ring (2..4 stages per warp) that still lets two CTAs share an SM
@@ -399,24 +393,9 @@ static int launch_one(MummuMoe* m, DecodeArgs& a, int n_experts_max, bool stream
             a.ring_depth = depth;
             LaunchScope scope(m, s, name);
             MUMMU_CUDA_TRY(allow_big_smem(decode_q4k_tma_kernel<NT, GATEUP>, m->cfg.device));
-            if (!GATEUP && pdl) {
-                // may start while the gate/up grid drains (it waits on the device before it reads hact)
-                cudaLaunchConfig_t cfg{};
-                cfg.gridDim = dim3((unsigned)(n_experts_max * a.ctas_per_expert), (unsigned)a.pass_split);
-                cfg.blockDim = dim3(DQ_THREADS);
-                cfg.dynamicSmemBytes = smem;
-                cfg.stream = s;
-                cudaLaunchAttribute attr[1];
-                attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-                attr[0].val.programmaticStreamSerializationAllowed = 1;
-                cfg.attrs = attr;
-                cfg.numAttrs = 1;
-                MUMMU_CUDA_TRY(cudaLaunchKernelEx(&cfg, decode_q4k_tma_kernel<NT, GATEUP>, a, *map0, *map1));
-            } else {
-                decode_q4k_tma_kernel<NT, GATEUP><<<dim3((unsigned)(n_experts_max * a.ctas_per_expert), (unsigned)a.pass_split), DQ_THREADS, smem, s>>>(a, *map0, *map1);
-            }
-            MUMMU_CUDA_TRY(cudaGetLastError());
-            if (used_tma) *used_tma = true;
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m) && !GATEUP, decode_q4k_tma_kernel<NT, GATEUP>,
+                                        dim3((unsigned)(n_experts_max * a.ctas_per_expert), (unsigned)a.pass_split), DQ_THREADS,
+                                        smem, s, a, *map0, *map1));
             return MUMMU_OK;
         }
     }
@@ -428,8 +407,8 @@ static int launch_one(MummuMoe* m, DecodeArgs& a, int n_experts_max, bool stream
     }
     LaunchScope scope(m, s, name);
     MUMMU_CUDA_TRY(allow_big_smem(decode_q4k_kernel<NT, GATEUP>, m->cfg.device));
-    decode_q4k_kernel<NT, GATEUP><<<n_experts_max * a.ctas_per_expert, DQ_THREADS, smem, s>>>(a);
-    MUMMU_CUDA_TRY(cudaGetLastError());
+    MUMMU_CUDA_TRY(launch_chain(chain_early(m), decode_q4k_kernel<NT, GATEUP>, dim3((unsigned)(n_experts_max * a.ctas_per_expert)),
+                                DQ_THREADS, smem, s, a));
     return MUMMU_OK;
 }
 
@@ -491,17 +470,9 @@ int launch_decode_q4k_rows(MummuMoe* m, const void* x, const int32_t* row_token,
     g.out = m->hact;
     g.rows_per_expert = c.inter;
     g.status = m->status;
-    // Programmatic dependent launch of the down kernel behind gate/up (measured: 2 % of the layer
-    // at T=64, 6-8 % at T=8..32; MUMMU_CUDA_DECODE_NO_PDL=1 turns it off); profiling brackets
-    // every launch with events, which would serialise the pair anyway.
-    const bool want_pdl = !m->sw.decode_no_pdl && !m->prof.enabled;
-    g.pdl = want_pdl ? 1 : 0;
-    bool g_tma = false;
-    int rc = nt2 ? launch_one<2, true>(m, g, experts_est, g_stream, s, "q4k_gate_up", false, &g_tma)
-                 : launch_one<1, true>(m, g, experts_est, g_stream, s, "q4k_gate_up", false, &g_tma);
+    int rc = nt2 ? launch_one<2, true>(m, g, experts_est, g_stream, s, "q4k_gate_up")
+                 : launch_one<1, true>(m, g, experts_est, g_stream, s, "q4k_gate_up");
     if (rc) return rc;
-    // profiling brackets every launch with events, which would serialise the pair anyway
-    const bool pdl = g_tma && want_pdl;
 
     DecodeArgs d{};
     d.x = (const __half*)m->hact;
@@ -518,13 +489,12 @@ int launch_decode_q4k_rows(MummuMoe* m, const void* x, const int32_t* row_token,
     d.n_rt = c.hidden / 32;
     bool d_stream;
     plan(m->sw, d, experts_est, rows_total, nt2 ? 2 : 1, d_stream);
-    d.pdl = pdl ? 1 : 0;
     d.ld_out = c.hidden;
     d.out = ys;
     d.rows_per_expert = c.hidden;
     d.status = m->status;
-    return nt2 ? launch_one<2, false>(m, d, experts_est, d_stream, s, "q4k_down", pdl)
-               : launch_one<1, false>(m, d, experts_est, d_stream, s, "q4k_down", pdl);
+    return nt2 ? launch_one<2, false>(m, d, experts_est, d_stream, s, "q4k_down")
+               : launch_one<1, false>(m, d, experts_est, d_stream, s, "q4k_down");
 }
 
 int launch_decode_q4k(MummuMoe* m, const void* x, int64_t tokens, int top_k, cudaStream_t s) {

@@ -29,7 +29,6 @@ struct DecodeArgs {
     void* out;                  // gate/up: __half hact; down: float ys
     int rows_per_expert;        // weight rows per expert (TMA row coordinate)
     int ring_depth;             // TMA stages per warp
-    int pdl;                    // this launch is one of a programmatically dependent pair
     int pass_split;             // CTAs sharing the passes of an expert (grid y)
     int32_t* status;            // handle's device status word
 };

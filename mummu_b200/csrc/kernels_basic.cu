@@ -291,24 +291,11 @@ __global__ void __launch_bounds__(R_THREADS) router_kernel(RouterArgs a) {
     const int t0 = blockIdx.y * TT;
     const TX* x = reinterpret_cast<const TX*>(a.x);
 
+    if constexpr (!TR) pdl_enter();
     if constexpr (TR) {
         const int steps = H >> 3;                              // i = 0 .. steps-1, row h = 8 i + j
-        // x first (kept in registers while W streams in), then W eight rows per thread at a time
-        // with all loads issued before the first store: the block's critical path is L2 latency
-        constexpr int XU = TT;                                // 16-byte groups per thread up to H = 2048
-        uint4 xv[XU];
-        const int xgroups = TT * steps;
-#pragma unroll
-        for (int u = 0; u < XU; ++u) {
-            const int idx = tid + u * R_THREADS;
-            xv[u] = make_uint4(0, 0, 0, 0);
-            if (idx < xgroups && idx < XU * R_THREADS) {
-                const int tt = idx / steps, i = idx - tt * steps;
-                if (t0 + tt < a.T) xv[u] = *reinterpret_cast<const uint4*>(x + (size_t)(t0 + tt) * H + (size_t)i * 8);
-            }
-        }
-        // W: the slice's image lies contiguous in global memory; one bulk copy by the copy engine
-        // (issued first, above the x loads would be even better, but x needs no barrier)
+        // W: the slice's image lies contiguous in global memory; one bulk copy by the copy engine, asked for
+        // while the kernel before still drains (nothing in a call writes the weights)
         const uint32_t bar = smem_u32(&w_bar);
         const uint32_t w_bytes = (uint32_t)(64 * S * 4);
         if (tid == 0) {
@@ -320,6 +307,20 @@ __global__ void __launch_bounds__(R_THREADS) router_kernel(RouterArgs a) {
                     smem_u32(Ws)),
                 "l"(a.wt + (size_t)blockIdx.x * 64 * S), "r"(w_bytes), "r"(bar)
                 : "memory");
+        }
+        pdl_enter();
+        // x, kept in registers while W streams in
+        constexpr int XU = TT;                                // 16-byte groups per thread up to H = 2048
+        uint4 xv[XU];
+        const int xgroups = TT * steps;
+#pragma unroll
+        for (int u = 0; u < XU; ++u) {
+            const int idx = tid + u * R_THREADS;
+            xv[u] = make_uint4(0, 0, 0, 0);
+            if (idx < xgroups && idx < XU * R_THREADS) {
+                const int tt = idx / steps, i = idx - tt * steps;
+                if (t0 + tt < a.T) xv[u] = *reinterpret_cast<const uint4*>(x + (size_t)(t0 + tt) * H + (size_t)i * 8);
+            }
         }
 #pragma unroll
         for (int u = 0; u < XU; ++u) {
@@ -496,6 +497,7 @@ __global__ void __launch_bounds__(e_pad * 8 * SPLIT) router_wide_kernel(RouterAr
     const int tid = threadIdx.x, nthreads = blockDim.x;
     const int t0 = blockIdx.x * RW_TT;
     const TX* x = reinterpret_cast<const TX*>(a.x);
+    pdl_enter();
     for (int tt = 0; tt < RW_TT; ++tt) {
         const int t = t0 + tt;
         for (int k = tid; k < H8; k += nthreads)
@@ -712,6 +714,7 @@ __global__ void __launch_bounds__(256, 2) router_tile_kernel(RouterArgs a) {
     const int t0 = blockIdx.x * TT;
     const TX* x = reinterpret_cast<const TX*>(a.x);
     const int chunks = H8 / RT_KC;
+    pdl_enter();
     // staging roles: thread -> (token, octet of the chunk) for x; four 16-byte pieces of the weights
     const int x_oc = tid & 7, x_t = tid >> 3;
     const bool x_role = x_t < TT;
@@ -854,10 +857,10 @@ static int launch_router_t(MummuMoe* m, RouterArgs& a, cudaStream_t s) {
         LaunchScope scope(m, s, "router");
         if (big) {
             MUMMU_CUDA_TRY(allow_big_smem(router_tile_kernel<TX, 8>, m->cfg.device));
-            router_tile_kernel<TX, 8><<<(a.T + 31) / 32, 256, smem, s>>>(a);
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m), router_tile_kernel<TX, 8>, dim3((a.T + 31) / 32), (unsigned)(256), smem, s, a));
         } else {
             MUMMU_CUDA_TRY(allow_big_smem(router_tile_kernel<TX, 4>, m->cfg.device));
-            router_tile_kernel<TX, 4><<<(a.T + 15) / 16, 256, smem, s>>>(a);
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m), router_tile_kernel<TX, 4>, dim3((a.T + 15) / 16), (unsigned)(256), smem, s, a));
         }
         MUMMU_CUDA_TRY(cudaGetLastError());
         return MUMMU_OK;
@@ -874,19 +877,19 @@ static int launch_router_t(MummuMoe* m, RouterArgs& a, cudaStream_t s) {
             switch (e_pad) {
                 case 32:
                     MUMMU_CUDA_TRY(allow_big_smem(router_wide_kernel<TX, 32, 16, 1>, m->cfg.device));
-                    router_wide_kernel<TX, 32, 16, 1><<<blocks, threads, smem, s>>>(a);
+                    MUMMU_CUDA_TRY(launch_chain(chain_early(m), router_wide_kernel<TX, 32, 16, 1>, dim3(blocks), (unsigned)(threads), smem, s, a));
                     break;
                 case 64:
                     MUMMU_CUDA_TRY(allow_big_smem(router_wide_kernel<TX, 64, 16, 1>, m->cfg.device));
-                    router_wide_kernel<TX, 64, 16, 1><<<blocks, threads, smem, s>>>(a);
+                    MUMMU_CUDA_TRY(launch_chain(chain_early(m), router_wide_kernel<TX, 64, 16, 1>, dim3(blocks), (unsigned)(threads), smem, s, a));
                     break;
                 case 96:
                     MUMMU_CUDA_TRY(allow_big_smem(router_wide_kernel<TX, 96, 8, 1>, m->cfg.device));
-                    router_wide_kernel<TX, 96, 8, 1><<<blocks, threads, smem, s>>>(a);
+                    MUMMU_CUDA_TRY(launch_chain(chain_early(m), router_wide_kernel<TX, 96, 8, 1>, dim3(blocks), (unsigned)(threads), smem, s, a));
                     break;
                 default:
                     MUMMU_CUDA_TRY(allow_big_smem(router_wide_kernel<TX, 128, 8, 1>, m->cfg.device));
-                    router_wide_kernel<TX, 128, 8, 1><<<blocks, threads, smem, s>>>(a);
+                    MUMMU_CUDA_TRY(launch_chain(chain_early(m), router_wide_kernel<TX, 128, 8, 1>, dim3(blocks), (unsigned)(threads), smem, s, a));
                     break;
             }
             MUMMU_CUDA_TRY(cudaGetLastError());
@@ -903,7 +906,7 @@ static int launch_router_t(MummuMoe* m, RouterArgs& a, cudaStream_t s) {
             dim3 grid_t(a.E / R_ES, (a.T + 3) / 4);
             LaunchScope scope(m, s, "router");
             MUMMU_CUDA_TRY(allow_big_smem(router_kernel<TX, 1, true>, m->cfg.device));
-            router_kernel<TX, 1, true><<<grid_t, R_THREADS, smem_t, s>>>(a);
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m), router_kernel<TX, 1, true>, dim3(grid_t), (unsigned)(R_THREADS), smem_t, s, a));
             MUMMU_CUDA_TRY(cudaGetLastError());
             return MUMMU_OK;
         }
@@ -918,15 +921,15 @@ static int launch_router_t(MummuMoe* m, RouterArgs& a, cudaStream_t s) {
     switch (tpt) {
         case 4:
             MUMMU_CUDA_TRY(allow_big_smem(router_kernel<TX, 4, false>, m->cfg.device));
-            router_kernel<TX, 4, false><<<grid, R_THREADS, smem, s>>>(a);
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m), router_kernel<TX, 4, false>, dim3(grid), (unsigned)(R_THREADS), smem, s, a));
             break;
         case 2:
             MUMMU_CUDA_TRY(allow_big_smem(router_kernel<TX, 2, false>, m->cfg.device));
-            router_kernel<TX, 2, false><<<grid, R_THREADS, smem, s>>>(a);
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m), router_kernel<TX, 2, false>, dim3(grid), (unsigned)(R_THREADS), smem, s, a));
             break;
         default:
             MUMMU_CUDA_TRY(allow_big_smem(router_kernel<TX, 1, false>, m->cfg.device));
-            router_kernel<TX, 1, false><<<grid, R_THREADS, smem, s>>>(a);
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m), router_kernel<TX, 1, false>, dim3(grid), (unsigned)(R_THREADS), smem, s, a));
             break;
     }
     MUMMU_CUDA_TRY(cudaGetLastError());
@@ -1151,6 +1154,7 @@ __global__ void __launch_bounds__(P_THREADS) permute_kernel(const int32_t* ids, 
     __shared__ int base_s;
     const int e = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_enter();
     // exclusive prefix of counts up to e
     // part: rows of experts before e (exclusive prefix).  nz: experts that come before e in the
     // work order "most rows first, then lower id" - longest jobs are scheduled first so that the
@@ -1244,6 +1248,7 @@ __global__ void __launch_bounds__(PS_WARPS * 32) permute_count_kernel(const int3
     extern __shared__ int32_t s_tbl[];                           // [PS_WARPS][E]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int32_t* tbl = s_tbl + warp * E;
+    pdl_enter();
     for (int e = lane; e < E; e += 32) tbl[e] = 0;
     __syncwarp();
     const int64_t first = ((int64_t)blockIdx.x * PS_WARPS + warp) * PS_PAIRS_PER_WARP;
@@ -1264,6 +1269,7 @@ __global__ void __launch_bounds__(32) permute_scan_kernel(const int32_t* __restr
                                                           int32_t* __restrict__ whist, int32_t* offsets, int32_t* active,
                                                           int32_t* n_active) {
     const int e = blockIdx.x, lane = threadIdx.x;
+    pdl_enter();
     const int mine = counts[e];
     int before = 0, nz = 0;
     for (int i = lane; i < E; i += 32) {
@@ -1306,6 +1312,7 @@ __global__ void __launch_bounds__(PS_WARPS * 32) permute_scatter_kernel(const in
     extern __shared__ int32_t s_tbl[];                           // [PS_WARPS][E]: next row of the expert for this warp
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int32_t* nxt = s_tbl + warp * E;
+    pdl_enter();
     const int32_t* base = whist + ((int64_t)blockIdx.x * PS_WARPS + warp) * E;
     for (int e = lane; e < E; e += 32) nxt[e] = base[e];
     __syncwarp();
@@ -1337,16 +1344,16 @@ int launch_permute(MummuMoe* m, const int32_t* ids, int64_t tokens, int top_k,
     // three launches cost about 15 us of launch latency: they pay from about 64 K pairs on
     if (n >= 65536 && m->whist && blocks * PS_WARPS * E <= m->whist_elems && tbl_bytes <= 48 * 1024) {
         LaunchScope scope(m, s, "permute");
-        permute_count_kernel<<<(unsigned)blocks, PS_WARPS * 32, tbl_bytes, s>>>(ids, n, E, m->whist);
-        permute_scan_kernel<<<E, 32, 0, s>>>(counts, E, blocks * PS_WARPS, m->whist, offsets, m->active, m->n_active);
-        permute_scatter_kernel<<<(unsigned)blocks, PS_WARPS * 32, tbl_bytes, s>>>(ids, n, top_k, E, m->whist, row_token, pos);
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m), permute_count_kernel, dim3((unsigned)blocks), (unsigned)(PS_WARPS * 32), tbl_bytes, s, ids, n, E, m->whist));
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m), permute_scan_kernel, dim3(E), (unsigned)(32), 0, s, counts, E, blocks * PS_WARPS, m->whist, offsets, m->active, m->n_active));
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m), permute_scatter_kernel, dim3((unsigned)blocks), (unsigned)(PS_WARPS * 32), tbl_bytes, s, ids, n, top_k, E, m->whist, row_token, pos));
         MUMMU_CUDA_TRY(cudaGetLastError());
         return MUMMU_OK;
     }
     LaunchScope scope(m, s, "permute");
-    permute_kernel<<<m->cfg.experts, P_THREADS, 0, s>>>(ids, tokens * top_k, top_k, m->cfg.experts,
+    MUMMU_CUDA_TRY(launch_chain(chain_early(m), permute_kernel, dim3(m->cfg.experts), (unsigned)(P_THREADS), 0, s, ids, tokens * top_k, top_k, m->cfg.experts,
                                                         counts, offsets, row_token, pos, m->active,
-                                                        m->n_active);
+                                                        m->n_active));
     MUMMU_CUDA_TRY(cudaGetLastError());
     return MUMMU_OK;
 }
@@ -1361,6 +1368,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const TY* ys, const int32_
     int32_t* s_pos = reinterpret_cast<int32_t*>(smem_raw);
     float* s_w = reinterpret_cast<float*>(s_pos + top_k);
     const int64_t t = blockIdx.x;
+    pdl_enter();
     for (int r = threadIdx.x; r < top_k; r += blockDim.x) {
         int id = ids[t * top_k + r];
         int rank = 0;
@@ -1411,6 +1419,7 @@ __global__ void __launch_bounds__(256) combine_vec8_kernel(const TY* ys, const i
     int32_t* s_pos = reinterpret_cast<int32_t*>(smem_raw);
     float* s_w = reinterpret_cast<float*>(s_pos + top_k);
     const int64_t t = blockIdx.x;
+    pdl_enter();
     for (int r = threadIdx.x; r < top_k; r += blockDim.x) {
         int id = ids[t * top_k + r];
         int rank = 0;
@@ -1459,16 +1468,16 @@ static int launch_combine_y(MummuMoe* m, const void* ys, const int32_t* ids, con
     if (vec) {
         switch (m->cfg.act_dtype) {
             case MUMMU_F32:
-                if (tokens < 128) combine_vec8_kernel<TY, float, 8><<<grid, vthreads, smem, s>>>((const TY*)ys, ids, w, pos, top_k, H, (float*)out);
-                else combine_vec8_kernel<TY, float, 4><<<grid, vthreads, smem, s>>>((const TY*)ys, ids, w, pos, top_k, H, (float*)out);
+                if (tokens < 128) MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_vec8_kernel<TY, float, 8>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (float*)out));
+                else MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_vec8_kernel<TY, float, 4>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (float*)out));
                 break;
             case MUMMU_F16:
-                if (tokens < 128) combine_vec8_kernel<TY, __half, 8><<<grid, vthreads, smem, s>>>((const TY*)ys, ids, w, pos, top_k, H, (__half*)out);
-                else combine_vec8_kernel<TY, __half, 4><<<grid, vthreads, smem, s>>>((const TY*)ys, ids, w, pos, top_k, H, (__half*)out);
+                if (tokens < 128) MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_vec8_kernel<TY, __half, 8>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__half*)out));
+                else MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_vec8_kernel<TY, __half, 4>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__half*)out));
                 break;
             case MUMMU_BF16:
-                if (tokens < 128) combine_vec8_kernel<TY, __nv_bfloat16, 8><<<grid, vthreads, smem, s>>>((const TY*)ys, ids, w, pos, top_k, H, (__nv_bfloat16*)out);
-                else combine_vec8_kernel<TY, __nv_bfloat16, 4><<<grid, vthreads, smem, s>>>((const TY*)ys, ids, w, pos, top_k, H, (__nv_bfloat16*)out);
+                if (tokens < 128) MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_vec8_kernel<TY, __nv_bfloat16, 8>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__nv_bfloat16*)out));
+                else MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_vec8_kernel<TY, __nv_bfloat16, 4>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__nv_bfloat16*)out));
                 break;
         }
         MUMMU_CUDA_TRY(cudaGetLastError());
@@ -1476,13 +1485,13 @@ static int launch_combine_y(MummuMoe* m, const void* ys, const int32_t* ids, con
     }
     switch (m->cfg.act_dtype) {
         case MUMMU_F32:
-            combine_kernel<TY, float><<<grid, 256, smem, s>>>((const TY*)ys, ids, w, pos, top_k, H, (float*)out);
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_kernel<TY, float>, dim3(grid), (unsigned)(256), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (float*)out));
             break;
         case MUMMU_F16:
-            combine_kernel<TY, __half><<<grid, 256, smem, s>>>((const TY*)ys, ids, w, pos, top_k, H, (__half*)out);
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_kernel<TY, __half>, dim3(grid), (unsigned)(256), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__half*)out));
             break;
         case MUMMU_BF16:
-            combine_kernel<TY, __nv_bfloat16><<<grid, 256, smem, s>>>((const TY*)ys, ids, w, pos, top_k, H, (__nv_bfloat16*)out);
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_kernel<TY, __nv_bfloat16>, dim3(grid), (unsigned)(256), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__nv_bfloat16*)out));
             break;
     }
     MUMMU_CUDA_TRY(cudaGetLastError());
@@ -1697,6 +1706,7 @@ __global__ void __launch_bounds__(FS_ROWS) f32_stream_kernel(SimtArgs a) {
     float* ws = reinterpret_cast<float*>(smem_raw);                   // [FS_STAGES][128 weight rows][FS_PITCH]
     float* xs = ws + FS_STAGES * FS_ROWS * FS_PITCH;                  // [FS_STAGES][R][FS_BK]
     const int e = a.expert_single >= 0 ? a.expert_single : (int)blockIdx.z;
+    pdl_enter();
     const int cnt = a.counts ? a.counts[e] : a.rows_single;
     const int m0 = blockIdx.y * R;
     if (m0 >= cnt) return;
@@ -1795,10 +1805,10 @@ static int f32_stream_launch(MummuMoe* m, SimtArgs& a, int experts, int64_t max_
     LaunchScope scope(m, s, name);
     if (r16) {
         MUMMU_CUDA_TRY(allow_big_smem(f32_stream_kernel<16, GATEUP>, m->cfg.device));
-        f32_stream_kernel<16, GATEUP><<<grid, FS_ROWS, fs_smem_bytes<16>(), s>>>(a);
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m), f32_stream_kernel<16, GATEUP>, dim3(grid), (unsigned)(FS_ROWS), fs_smem_bytes<16>(), s, a));
     } else {
         MUMMU_CUDA_TRY(allow_big_smem(f32_stream_kernel<8, GATEUP>, m->cfg.device));
-        f32_stream_kernel<8, GATEUP><<<grid, FS_ROWS, fs_smem_bytes<8>(), s>>>(a);
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m), f32_stream_kernel<8, GATEUP>, dim3(grid), (unsigned)(FS_ROWS), fs_smem_bytes<8>(), s, a));
     }
     MUMMU_CUDA_TRY(cudaGetLastError());
     return MUMMU_OK;

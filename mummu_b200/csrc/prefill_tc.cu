@@ -231,14 +231,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + TC_STAGES);
     const uint32_t tfull0 = smem_u32(bars + 2 * TC_STAGES), tempty0 = smem_u32(bars + 2 * TC_STAGES + 2);
 
-    // tile prefix over experts (every CTA builds the same list)
     if (tid == 0) {
-        int acc = 0;
-        for (int e = 0; e < a.E; ++e) {
-            tile_start[e] = acc;
-            acc += ((a.counts[e] + TC_BM - 1) / TC_BM) * a.n_tiles;
-        }
-        tile_start[a.E] = acc;
         *abort_flag = 0;
         for (int s = 0; s < TC_STAGES; ++s) {
             mbar_init(full0 + 8 * s, 1);
@@ -254,6 +247,24 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     if (warp == 1) {
         tmem_alloc(smem_u32(tmem_slot), TC_TMEM_COLS);
         tmem_relinquish();
+    }
+    pdl_enter();
+    // tile prefix over experts (every CTA builds the same list): 32 experts at a time, prefix by shuffles
+    if (warp == 2) {
+        int acc = 0;
+        for (int e0 = 0; e0 < a.E; e0 += 32) {
+            const int e = e0 + lane;
+            const int c = e < a.E ? ((a.counts[e] + TC_BM - 1) / TC_BM) * a.n_tiles : 0;
+            int incl = c;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int up = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+                if (lane >= off) incl += up;
+            }
+            if (e < a.E) tile_start[e] = acc + incl - c;
+            acc += __shfl_sync(0xFFFFFFFFu, incl, 31);
+        }
+        if (lane == 0) tile_start[a.E] = acc;
     }
     tc_fence_before();
     __syncthreads();
@@ -408,6 +419,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         tmem_alloc_pair(smem_u32(tmem_slot), TC_TMEM_COLS);
         tmem_relinquish_pair();
     }
+    pdl_enter();
     if (warp == 2) {
         int acc = 0;
         for (int e0 = 0; e0 < a.E; e0 += 32) {
@@ -540,6 +552,7 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restric
                                                           uint4* __restrict__ xs, int64_t rows, int vec_per_row) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    pdl_enter();
     for (int64_t p = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); p < rows; p += warps) {
         const uint4* src = x + (size_t)row_token[p] * vec_per_row;
         uint4* dst = xs + (size_t)p * vec_per_row;
@@ -655,12 +668,12 @@ static int launch_tc_typed(MummuMoe* m, const void* xs, int64_t rows_cap, int64_
     if (pair) {
         MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_pair_kernel<TIN, TIN, true>, c.device));
         LaunchScope scope(m, s, "tc_gate_up");
-        grouped_gemm_pair_kernel<TIN, TIN, true><<<sms & ~1, TC_THREADS, smem_pair, s>>>(map_x, map_g, map_u, g);
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m), grouped_gemm_pair_kernel<TIN, TIN, true>, dim3(sms & ~1), (unsigned)(TC_THREADS), smem_pair, s, map_x, map_g, map_u, g));
         MUMMU_CUDA_TRY(cudaGetLastError());
     } else {
         MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_tc_kernel<TIN, TIN, true>, c.device));
         LaunchScope scope(m, s, "tc_gate_up");
-        grouped_gemm_tc_kernel<TIN, TIN, true><<<sms, TC_THREADS, smem, s>>>(map_x, map_g, map_u, g);
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m), grouped_gemm_tc_kernel<TIN, TIN, true>, dim3(sms), (unsigned)(TC_THREADS), smem, s, map_x, map_g, map_u, g));
         MUMMU_CUDA_TRY(cudaGetLastError());
     }
     TcArgs d{};
@@ -687,13 +700,13 @@ static int launch_tc_typed(MummuMoe* m, const void* xs, int64_t rows_cap, int64_
     LaunchScope scope(m, s, "tc_down");
     if (pair && ys_dtype != MUMMU_F32) {
         MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_pair_kernel<TIN, TIN, false>, c.device));
-        grouped_gemm_pair_kernel<TIN, TIN, false><<<sms & ~1, TC_THREADS, smem_pair, s>>>(map_h, map_d, map_d, d);
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m), grouped_gemm_pair_kernel<TIN, TIN, false>, dim3(sms & ~1), (unsigned)(TC_THREADS), smem_pair, s, map_h, map_d, map_d, d));
     } else if (ys_dtype == MUMMU_F32) {
         MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_tc_kernel<TIN, float, false>, c.device));
-        grouped_gemm_tc_kernel<TIN, float, false><<<sms, TC_THREADS, smem, s>>>(map_h, map_d, map_d, d);
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m), grouped_gemm_tc_kernel<TIN, float, false>, dim3(sms), (unsigned)(TC_THREADS), smem, s, map_h, map_d, map_d, d));
     } else {
         MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_tc_kernel<TIN, TIN, false>, c.device));
-        grouped_gemm_tc_kernel<TIN, TIN, false><<<sms, TC_THREADS, smem, s>>>(map_h, map_d, map_d, d);
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m), grouped_gemm_tc_kernel<TIN, TIN, false>, dim3(sms), (unsigned)(TC_THREADS), smem, s, map_h, map_d, map_d, d));
     }
     MUMMU_CUDA_TRY(cudaGetLastError());
     return MUMMU_OK;
@@ -729,6 +742,7 @@ struct ExpandBanks {
 __global__ void __launch_bounds__(256) q4k_expand_f16_kernel(ExpandBanks banks, int blocks_per_expert,
                                                              const int32_t* __restrict__ counts) {
     const int e = blockIdx.y;
+    pdl_enter();
     if (counts[e] == 0) return;                                  // nobody routed here this call
     const int lane = threadIdx.x & 31;
     const int j = lane >> 2, chunk = j >> 1, b0 = (lane & 3) * 8;
@@ -807,7 +821,7 @@ int launch_experts_q4k_tc(MummuMoe* m, const void* xs, int64_t rows_cap, int64_t
         }
         const int blocks_per_expert = (int)((int64_t)c.inter * c.hidden / 256);
         const dim3 grid((unsigned)((blocks_per_expert + QE_PER_CTA - 1) / QE_PER_CTA), (unsigned)c.experts_local, 3);
-        q4k_expand_f16_kernel<<<grid, 256, 0, s>>>(eb, blocks_per_expert, counts);
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m), q4k_expand_f16_kernel, dim3(grid), (unsigned)(256), 0, s, eb, blocks_per_expert, counts));
         MUMMU_CUDA_TRY(cudaGetLastError());
     }
     const void* banks[3] = {owner->wexp[0], owner->wexp[1], owner->wexp[2]};
@@ -820,7 +834,7 @@ int launch_gather_rows(MummuMoe* m, const void* x, const int32_t* row_token, voi
     const int vec = m->cfg.hidden * 2 / 16;
     int64_t blocks = rows < 8 ? 1 : (rows / 8 < 148 * 8 ? (rows + 7) / 8 : 148 * 8);     // a warp per row
     LaunchScope scope(m, s, "gather_rows");
-    gather_rows_kernel<<<(unsigned)blocks, 256, 0, s>>>((const uint4*)x, row_token, (uint4*)xs, rows, vec);
+    MUMMU_CUDA_TRY(launch_chain(chain_early(m), gather_rows_kernel, dim3((unsigned)blocks), (unsigned)(256), 0, s, (const uint4*)x, row_token, (uint4*)xs, rows, vec));
     MUMMU_CUDA_TRY(cudaGetLastError());
     return MUMMU_OK;
 }

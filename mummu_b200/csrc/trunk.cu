@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(512) add_rms_kernel(__half* x, const __half* y
     __shared__ float s_red[16];
     extern __shared__ __align__(16) float s_row[];
     const int slot = blockIdx.x;
+    pdl_enter();
     float ss = 0.0f;
     for (int k = threadIdx.x * 4; k < H; k += blockDim.x * 4) {
         float4 v = load_h4(x + (size_t)slot * H + k);
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(256) gemv_f16_kernel(const __half* __restrict_
     const bool rows_ok = row0 + 16 <= N;
     const __half* wa = W + (size_t)(row0 + g) * K;
     const __half* wb = wa + (size_t)8 * K;
+    pdl_enter();
     float acc[NTT][4];
 #pragma unroll
     for (int nt = 0; nt < NTT; ++nt)
@@ -207,6 +209,7 @@ __global__ void __launch_bounds__(512) qk_norm_rope_kernel(const float* part, in
     extern __shared__ __align__(16) float s_v[];
     __shared__ float s_red[16];
     const int slot = blockIdx.x, which = blockIdx.y;
+    pdl_enter();
     const int nq = heads * hd, nkv = kv_heads * hd, N = nq + 2 * nkv;
     const int n0 = which == 0 ? 0 : (which == 1 ? nq : nq + nkv), nn = which == 0 ? nq : nkv;
     float ss = 0.0f;
@@ -261,6 +264,7 @@ __global__ void __launch_bounds__(128) decode_attn_kernel(const __half* q, const
     extern __shared__ float s_attn[];               // scores [chunk] | per-warp value sums [4][hd]
     __shared__ float s_red[4];
     const int head = blockIdx.x, slot = blockIdx.y, sp = blockIdx.z;
+    pdl_enter();
     const int pos = min(positions[slot], key_len - 1);
     const int chunk = (key_len + splits - 1) / splits;
     const int lo = sp * chunk, hi = min(pos + 1, lo + chunk);
@@ -376,6 +380,7 @@ __global__ void __launch_bounds__(128) decode_attn_kernel(const __half* q, const
 
 __global__ void __launch_bounds__(128) attn_combine_kernel(const float* apart, __half* ctx, int heads, int hd, int splits) {
     const int head = blockIdx.x, slot = blockIdx.y;
+    pdl_enter();
     __shared__ float s_w[TR_MAX_SPLITS + 1];
     const float* base = apart + ((size_t)slot * heads + head) * splits * (hd + 2);
     if (threadIdx.x < 32) {                          // splits <= 32: a lane each
@@ -415,6 +420,7 @@ __global__ void __launch_bounds__(512) residual_rms_kernel(__half* x, const floa
     __shared__ float s_red[16];
     extern __shared__ __align__(16) float s_row[];
     const int slot = blockIdx.x;
+    pdl_enter();
     float ss = 0.0f;
     for (int k = threadIdx.x * 4; k < H; k += blockDim.x * 4) {
         const float4 a = load_h4(x + (size_t)slot * H + k);
@@ -432,6 +438,7 @@ __global__ void __launch_bounds__(512) residual_rms_kernel(__half* x, const floa
 
 __global__ void __launch_bounds__(256) embed_kernel(const __half* embed, const int32_t* tokens, __half* x, int H, int vocab) {
     const int slot = blockIdx.x;
+    pdl_enter();
     int tok = tokens[slot];
     tok = tok < 0 ? 0 : (tok >= vocab ? vocab - 1 : tok);
     const uint4* src = reinterpret_cast<const uint4*>(embed + (size_t)tok * H);
@@ -444,6 +451,7 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float* logits, int V
     __shared__ float s_v[32];
     __shared__ int s_i[32];
     const int slot = blockIdx.x;
+    pdl_enter();
     const float* row = logits + (size_t)slot * V;
     float bv = -FLT_MAX;
     int bi = 0x7FFFFFFF;
@@ -642,7 +650,7 @@ static int gemv(MummuTrunk* t, const __half* W, const __half* x, float* part, in
     do {                                                                                                        \
         const size_t smem = (size_t)8 * NTT * (512 + 32) * sizeof(__half);                                      \
         MUMMU_CUDA_TRY(allow_big_smem(gemv_f16_kernel<NTT>, t->cfg.device));                                    \
-        gemv_f16_kernel<NTT><<<grid, 256, smem, s>>>(W, x, part, N, K, k_per_block, B);                         \
+        MUMMU_CUDA_TRY(launch_chain(true, gemv_f16_kernel<NTT>, dim3(grid), (unsigned)(256), smem, s, W, x, part, N, K, k_per_block, B));                         \
     } while (0)
     if (ntt <= 1) MUMMU_GEMV(1);
     else if (ntt <= 2) MUMMU_GEMV(2);
@@ -823,7 +831,7 @@ int32_t mummu_trunk_embed(MummuTrunk* t, const int32_t* tokens, int32_t slots, v
     TrunkDevice guard(t->cfg.device);
     cudaStream_t s = stream ? (cudaStream_t)stream : t->stream;
     TrunkLaunch l(t);
-    embed_kernel<<<slots, 256, 0, s>>>(t->embed, tokens, (__half*)x, t->cfg.hidden, t->cfg.vocab);
+    MUMMU_CUDA_TRY(launch_chain(true, embed_kernel, dim3(slots), (unsigned)(256), 0, s, t->embed, tokens, (__half*)x, t->cfg.hidden, t->cfg.vocab));
     MUMMU_CUDA_TRY(cudaGetLastError());
     return MUMMU_OK;
 }
@@ -848,7 +856,7 @@ int32_t mummu_trunk_attention_step(MummuTrunk* t, int32_t layer, void* x, const 
     {   // x += y_prev (the previous layer's expert bank joins the residual stream); h = rmsnorm(x) * gamma_in
         TrunkLaunch l(t);
         MUMMU_CUDA_TRY(allow_big_smem(add_rms_kernel, c.device));
-        add_rms_kernel<<<slots, 512, (size_t)H * 4, s>>>((__half*)x, (const __half*)y_prev, g_in, t->h, H, c.rms_eps);
+        MUMMU_CUDA_TRY(launch_chain(true, add_rms_kernel, dim3(slots), (unsigned)(512), (size_t)H * 4, s, (__half*)x, (const __half*)y_prev, g_in, t->h, H, c.rms_eps));
         MUMMU_CUDA_TRY(cudaGetLastError());
     }
     const int ks_qkv = H >= 2048 ? 4 : (H >= 1024 ? 2 : 1);
@@ -859,9 +867,9 @@ int32_t mummu_trunk_attention_step(MummuTrunk* t, int32_t layer, void* x, const 
     {
         TrunkLaunch l(t);
         MUMMU_CUDA_TRY(allow_big_smem(qk_norm_rope_kernel, c.device));
-        qk_norm_rope_kernel<<<dim3(slots, 3), 512, (size_t)std::max(nq, nkv) * 4, s>>>(t->part, ks_qkv, slots, g_q, g_k, t->rope_cos, t->rope_sin,
+        MUMMU_CUDA_TRY(launch_chain(true, qk_norm_rope_kernel, dim3(dim3(slots, 3)), (unsigned)(512), (size_t)std::max(nq, nkv) * 4, s, t->part, ks_qkv, slots, g_q, g_k, t->rope_cos, t->rope_sin,
                                                                  positions, t->q, kc, vc, c.heads, c.kv_heads, c.head_dim,
-                                                                 c.max_ctx, c.rms_eps);
+                                                                 c.max_ctx, c.rms_eps));
         MUMMU_CUDA_TRY(cudaGetLastError());
     }
     // key splits: enough blocks to fill the GPU when few sequences decode, chunks of at most 1024 keys
@@ -873,14 +881,14 @@ int32_t mummu_trunk_attention_step(MummuTrunk* t, int32_t layer, void* x, const 
     {
         TrunkLaunch l(t);
         MUMMU_CUDA_TRY(allow_big_smem(decode_attn_kernel, c.device));
-        decode_attn_kernel<<<dim3(c.heads, slots, splits), 128, (size_t)(4 * c.head_dim + chunk) * 4, s>>>(
+        MUMMU_CUDA_TRY(launch_chain(true, decode_attn_kernel, dim3(dim3(c.heads, slots, splits)), (unsigned)(128), (size_t)(4 * c.head_dim + chunk) * 4, s, 
             t->q, kc, vc, positions, t->apart, c.heads, c.kv_heads, c.head_dim, c.max_ctx, key_len, splits,
-            1.0f / sqrtf((float)c.head_dim));
+            1.0f / sqrtf((float)c.head_dim)));
         MUMMU_CUDA_TRY(cudaGetLastError());
     }
     {
         TrunkLaunch l(t);
-        attn_combine_kernel<<<dim3(c.heads, slots), 128, 0, s>>>(t->apart, t->ctx, c.heads, c.head_dim, splits);
+        MUMMU_CUDA_TRY(launch_chain(true, attn_combine_kernel, dim3(dim3(c.heads, slots)), (unsigned)(128), 0, s, t->apart, t->ctx, c.heads, c.head_dim, splits));
         MUMMU_CUDA_TRY(cudaGetLastError());
     }
     const int ks_o = nq >= 2048 ? 8 : (nq >= 1024 ? 4 : 1);
@@ -888,7 +896,7 @@ int32_t mummu_trunk_attention_step(MummuTrunk* t, int32_t layer, void* x, const 
     {
         TrunkLaunch l(t);
         MUMMU_CUDA_TRY(allow_big_smem(residual_rms_kernel, c.device));
-        residual_rms_kernel<<<slots, 512, (size_t)H * 4, s>>>((__half*)x, t->part, ks_o, slots, g_post, (__half*)h2, H, c.rms_eps);
+        MUMMU_CUDA_TRY(launch_chain(true, residual_rms_kernel, dim3(slots), (unsigned)(512), (size_t)H * 4, s, (__half*)x, t->part, ks_o, slots, g_post, (__half*)h2, H, c.rms_eps));
         MUMMU_CUDA_TRY(cudaGetLastError());
     }
     return MUMMU_OK;
@@ -906,14 +914,14 @@ int32_t mummu_trunk_head(MummuTrunk* t, void* x, const void* y_prev, int32_t slo
     {
         TrunkLaunch l(t);
         MUMMU_CUDA_TRY(allow_big_smem(add_rms_kernel, c.device));
-        add_rms_kernel<<<slots, 512, (size_t)c.hidden * 4, s>>>((__half*)x, (const __half*)y_prev, t->final_norm, t->h, c.hidden,
-                                                                c.rms_eps);
+        MUMMU_CUDA_TRY(launch_chain(true, add_rms_kernel, dim3(slots), (unsigned)(512), (size_t)c.hidden * 4, s, (__half*)x, (const __half*)y_prev, t->final_norm, t->h, c.hidden,
+                                                                c.rms_eps));
         MUMMU_CUDA_TRY(cudaGetLastError());
     }
     if ((rc = gemv(t, t->lm_head, t->h, logits, c.vocab, c.hidden, 1, slots, s))) return rc;
     if (argmax) {
         TrunkLaunch l(t);
-        argmax_kernel<<<slots, 1024, 0, s>>>(logits, c.vocab, argmax);
+        MUMMU_CUDA_TRY(launch_chain(true, argmax_kernel, dim3(slots), (unsigned)(1024), 0, s, logits, c.vocab, argmax));
         MUMMU_CUDA_TRY(cudaGetLastError());
     }
     return MUMMU_OK;

@@ -54,3 +54,42 @@ def test_pair_gemm_against_the_single_cta_gemm(cuda_lib, dtype, H, I, E, K, T, s
     assert (whole[:part].float() - single.float()).abs().max().item() <= (2.0 ** -8 if dtype == "bf16" else 2.0 ** -10) * top
     assert torch.isfinite(whole.float()).all()
     m.close()
+
+
+@pytest.mark.parametrize("kv_heads", [4, 2])
+def test_static_step_over_split_keys_equals_the_growing_cache_step(cuda_lib, kv_heads):
+    """Sequences of very different lengths in one step: the key splits follow each sequence's own length (some
+    of them without a key), and the partials fold to the step of the growing-cache path.  Both round the same
+    16-bit activations; 2e-2 of the largest logit is the bar the model tests use."""
+    import torch
+    from mummu_b200 import _lib as L
+    from mummu_b200.olmoe import OlmoeConfig, OlmoeDecoder
+    cfg = OlmoeConfig(vocab_size=256, hidden_size=256, intermediate_size=256, num_hidden_layers=2,
+                      num_attention_heads=4, num_key_value_heads=kv_heads, num_experts=4, num_experts_per_tok=2)
+    lengths = [1, 31, 300, 639]
+    B, ctx = len(lengths), 640
+    dec = OlmoeDecoder(cfg, device=0, expert_dtype=L.Q4_K, max_batch=B, max_ctx=ctx)
+    if kv_heads != 4:                                  # random_init draws square k / v projections
+        dec.random_init(seed=1)
+        for lay in dec.layers:
+            n = kv_heads * cfg.head_dim
+            lay.update(k=lay["k"][:n].contiguous(), v=lay["v"][:n].contiguous(), k_norm=lay["k_norm"][:n].contiguous())
+    else:
+        dec.random_init(seed=1)
+    dec.embed.mul_(50.0)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    dec.k_cache.normal_(generator=g)
+    dec.v_cache.normal_(generator=g)
+    ids = torch.randint(0, cfg.vocab_size, (B, 1), generator=g, device="cuda")
+    state = dec.static_state(B, ctx)
+    for b in range(B):
+        dec.seed_static(state, b, lengths[b])
+    got = dec.forward_static(ids.to(torch.int32), torch.tensor(lengths, dtype=torch.int32, device="cuda"), state, ctx).clone()
+    for b in range(B):
+        dec.k_cache[:, 0].copy_(dec.k_cache[:, b].clone())
+        dec.v_cache[:, 0].copy_(dec.v_cache[:, b].clone())
+        want = dec.forward(ids[b:b + 1], lengths[b])
+        assert (got[b] - want[0]).abs().max().item() <= 2e-2 * want.abs().max().item(), lengths[b]
+        assert state.argmax[b].item() == got[b].argmax().item()
+    state.close()
+    dec.close()
