@@ -64,12 +64,26 @@ __global__ void __launch_bounds__(DQ_THREADS, 2) decode_q4k_kernel(DecodeArgs a)
     const int rt_end = min(a.n_rt, rt_begin + a.rb);
     const uint8_t* w0e = a.w0 + (size_t)e * a.expert_stride;
     const uint8_t* w1e = GATEUP ? a.w1 + (size_t)e * a.expert_stride : w0e;
+    auto load_pair = [&](UnitRegs (&un)[2], int rt, int sb) {
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+            const int row = GATEUP ? rt * 16 + g : rt * 32 + 16 * mt + g;
+            const uint8_t* row0 = (mt == 0 ? w0e : w1e) + (size_t)row * a.row_bytes + (size_t)sb * Q4K_BLOCK_BYTES;
+            load_unit(un[mt], row0, row0 + (size_t)8 * a.row_bytes, t);
+        }
+    };
+    // the first weights are on their way while the tokens are staged (one token: they are all the warp reads)
+    // (two token tiles leave no registers for that)
+    bool loaded = NT == 1 && warp_active && rt_begin + rg < rt_end;
+    UnitRegs early[NT == 1 ? 2 : 1];
+    if constexpr (NT == 1)
+        if (loaded) load_pair(early, rt_begin + rg, ks);
 
     for (int pass0 = 0; pass0 < cnt; pass0 += 8 * NT) {
         const int npass = min(8 * NT, cnt - pass0);
         const int nt_count = (npass + 7) >> 3;
         __syncthreads();   // previous pass finished reading the token tile
-        stage_token_tile<NT>(a, s_frag, s_sxh, base + pass0, npass, nt_count, tid);
+        stage_token_tile<NT>(a, s_frag, s_sxh, base + pass0, npass, tid);
         __syncthreads();
 
         int it = 0;
@@ -85,13 +99,14 @@ __global__ void __launch_bounds__(DQ_THREADS, 2) decode_q4k_kernel(DecodeArgs a)
 
             if (warp_active && rt < rt_end) {
                 for (int sb = ks; sb < nsb; sb += KS) {
-                    UnitRegs un[2];
-#pragma unroll
-                    for (int mt = 0; mt < 2; ++mt) {
-                        const int row = GATEUP ? rt * 16 + g : rt * 32 + 16 * mt + g;
-                        const uint8_t* row0 = (mt == 0 ? w0e : w1e) + (size_t)row * a.row_bytes +
-                                              (size_t)sb * Q4K_BLOCK_BYTES;
-                        load_unit(un[mt], row0, row0 + (size_t)8 * a.row_bytes, t);
+                    UnitRegs late[NT == 1 ? 1 : 2];
+                    UnitRegs* un = late;
+                    if constexpr (NT == 1) {
+                        if (!loaded) load_pair(early, rt, sb);
+                        loaded = false;
+                        un = early;
+                    } else {
+                        load_pair(late, rt, sb);
                     }
                     const uint32_t frag_addr = frag_base + (uint32_t)(((sb * NT * 64 + g) * 4 + t) * 16);
                     const uint32_t sxh_addr = sxh_base + (uint32_t)((((sb * NT * 8 + g) * 8) + 2 * t) * 2);
@@ -342,7 +357,7 @@ decode_q4k_tma_kernel(DecodeArgs a, const __grid_constant__ CUtensorMap map0, co
         const int npass = min(8 * NT, cnt - pass0);
         const int nt_count = (npass + 7) >> 3;
         __syncthreads();
-        stage_token_tile<NT>(a, s_frag, s_sxh, base + pass0, npass, nt_count, tid);
+        stage_token_tile<NT>(a, s_frag, s_sxh, base + pass0, npass, tid);
         __syncthreads();
 
         if (NT == 1 || nt_count == 1)
