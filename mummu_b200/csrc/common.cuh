@@ -304,8 +304,10 @@ cudaError_t launch_chain(bool early, void (*kernel)(Params...), dim3 grid, unsig
     cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
-// profiling brackets every launch with events, which would serialise the chain anyway
-inline bool chain_early(const MummuMoe* m) { return !m->sw.decode_no_pdl && !m->prof.enabled; }
+// Profiling brackets every launch with events, which would serialise the chain anyway.  pairs: (token, slot) pairs of
+// the call, where the kernels run long: 777 tokens (6216 pairs) 916 -> 899 us with early launches, but 4096 tokens
+// (32768 pairs) 581 -> 588 us, so large calls are launched the ordinary way.
+inline bool chain_early(const MummuMoe* m, int64_t pairs = 0) { return !m->sw.decode_no_pdl && !m->prof.enabled && pairs < 16384; }
 
 // ---- kernels_basic.cu ----
 // where the fused grouping of a decode-sized router call writes (null = the handle's own scratch)

@@ -857,10 +857,10 @@ static int launch_router_t(MummuMoe* m, RouterArgs& a, cudaStream_t s) {
         LaunchScope scope(m, s, "router");
         if (big) {
             MUMMU_CUDA_TRY(allow_big_smem(router_tile_kernel<TX, 8>, m->cfg.device));
-            MUMMU_CUDA_TRY(launch_chain(chain_early(m), router_tile_kernel<TX, 8>, dim3((a.T + 31) / 32), (unsigned)(256), smem, s, a));
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m, (int64_t)a.T * a.k), router_tile_kernel<TX, 8>, dim3((a.T + 31) / 32), (unsigned)(256), smem, s, a));
         } else {
             MUMMU_CUDA_TRY(allow_big_smem(router_tile_kernel<TX, 4>, m->cfg.device));
-            MUMMU_CUDA_TRY(launch_chain(chain_early(m), router_tile_kernel<TX, 4>, dim3((a.T + 15) / 16), (unsigned)(256), smem, s, a));
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m, (int64_t)a.T * a.k), router_tile_kernel<TX, 4>, dim3((a.T + 15) / 16), (unsigned)(256), smem, s, a));
         }
         MUMMU_CUDA_TRY(cudaGetLastError());
         return MUMMU_OK;
@@ -1344,14 +1344,14 @@ int launch_permute(MummuMoe* m, const int32_t* ids, int64_t tokens, int top_k,
     // three launches cost about 15 us of launch latency: they pay from about 64 K pairs on
     if (n >= 65536 && m->whist && blocks * PS_WARPS * E <= m->whist_elems && tbl_bytes <= 48 * 1024) {
         LaunchScope scope(m, s, "permute");
-        MUMMU_CUDA_TRY(launch_chain(chain_early(m), permute_count_kernel, dim3((unsigned)blocks), (unsigned)(PS_WARPS * 32), tbl_bytes, s, ids, n, E, m->whist));
-        MUMMU_CUDA_TRY(launch_chain(chain_early(m), permute_scan_kernel, dim3(E), (unsigned)(32), 0, s, counts, E, blocks * PS_WARPS, m->whist, offsets, m->active, m->n_active));
-        MUMMU_CUDA_TRY(launch_chain(chain_early(m), permute_scatter_kernel, dim3((unsigned)blocks), (unsigned)(PS_WARPS * 32), tbl_bytes, s, ids, n, top_k, E, m->whist, row_token, pos));
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m, n), permute_count_kernel, dim3((unsigned)blocks), (unsigned)(PS_WARPS * 32), tbl_bytes, s, ids, n, E, m->whist));
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m, n), permute_scan_kernel, dim3(E), (unsigned)(32), 0, s, counts, E, blocks * PS_WARPS, m->whist, offsets, m->active, m->n_active));
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m, n), permute_scatter_kernel, dim3((unsigned)blocks), (unsigned)(PS_WARPS * 32), tbl_bytes, s, ids, n, top_k, E, m->whist, row_token, pos));
         MUMMU_CUDA_TRY(cudaGetLastError());
         return MUMMU_OK;
     }
     LaunchScope scope(m, s, "permute");
-    MUMMU_CUDA_TRY(launch_chain(chain_early(m), permute_kernel, dim3(m->cfg.experts), (unsigned)(P_THREADS), 0, s, ids, tokens * top_k, top_k, m->cfg.experts,
+    MUMMU_CUDA_TRY(launch_chain(chain_early(m, n), permute_kernel, dim3(m->cfg.experts), (unsigned)(P_THREADS), 0, s, ids, tokens * top_k, top_k, m->cfg.experts,
                                                         counts, offsets, row_token, pos, m->active,
                                                         m->n_active));
     MUMMU_CUDA_TRY(cudaGetLastError());
@@ -1468,16 +1468,16 @@ static int launch_combine_y(MummuMoe* m, const void* ys, const int32_t* ids, con
     if (vec) {
         switch (m->cfg.act_dtype) {
             case MUMMU_F32:
-                if (tokens < 128) MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_vec8_kernel<TY, float, 8>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (float*)out));
-                else MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_vec8_kernel<TY, float, 4>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (float*)out));
+                if (tokens < 128) MUMMU_CUDA_TRY(launch_chain(chain_early(m, tokens * top_k), combine_vec8_kernel<TY, float, 8>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (float*)out));
+                else MUMMU_CUDA_TRY(launch_chain(chain_early(m, tokens * top_k), combine_vec8_kernel<TY, float, 4>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (float*)out));
                 break;
             case MUMMU_F16:
-                if (tokens < 128) MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_vec8_kernel<TY, __half, 8>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__half*)out));
-                else MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_vec8_kernel<TY, __half, 4>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__half*)out));
+                if (tokens < 128) MUMMU_CUDA_TRY(launch_chain(chain_early(m, tokens * top_k), combine_vec8_kernel<TY, __half, 8>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__half*)out));
+                else MUMMU_CUDA_TRY(launch_chain(chain_early(m, tokens * top_k), combine_vec8_kernel<TY, __half, 4>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__half*)out));
                 break;
             case MUMMU_BF16:
-                if (tokens < 128) MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_vec8_kernel<TY, __nv_bfloat16, 8>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__nv_bfloat16*)out));
-                else MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_vec8_kernel<TY, __nv_bfloat16, 4>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__nv_bfloat16*)out));
+                if (tokens < 128) MUMMU_CUDA_TRY(launch_chain(chain_early(m, tokens * top_k), combine_vec8_kernel<TY, __nv_bfloat16, 8>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__nv_bfloat16*)out));
+                else MUMMU_CUDA_TRY(launch_chain(chain_early(m, tokens * top_k), combine_vec8_kernel<TY, __nv_bfloat16, 4>, dim3(grid), (unsigned)(vthreads), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__nv_bfloat16*)out));
                 break;
         }
         MUMMU_CUDA_TRY(cudaGetLastError());
@@ -1485,13 +1485,13 @@ static int launch_combine_y(MummuMoe* m, const void* ys, const int32_t* ids, con
     }
     switch (m->cfg.act_dtype) {
         case MUMMU_F32:
-            MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_kernel<TY, float>, dim3(grid), (unsigned)(256), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (float*)out));
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m, tokens * top_k), combine_kernel<TY, float>, dim3(grid), (unsigned)(256), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (float*)out));
             break;
         case MUMMU_F16:
-            MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_kernel<TY, __half>, dim3(grid), (unsigned)(256), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__half*)out));
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m, tokens * top_k), combine_kernel<TY, __half>, dim3(grid), (unsigned)(256), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__half*)out));
             break;
         case MUMMU_BF16:
-            MUMMU_CUDA_TRY(launch_chain(chain_early(m), combine_kernel<TY, __nv_bfloat16>, dim3(grid), (unsigned)(256), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__nv_bfloat16*)out));
+            MUMMU_CUDA_TRY(launch_chain(chain_early(m, tokens * top_k), combine_kernel<TY, __nv_bfloat16>, dim3(grid), (unsigned)(256), smem, s, (const TY*)ys, ids, w, pos, top_k, H, (__nv_bfloat16*)out));
             break;
     }
     MUMMU_CUDA_TRY(cudaGetLastError());

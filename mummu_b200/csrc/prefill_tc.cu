@@ -668,12 +668,12 @@ static int launch_tc_typed(MummuMoe* m, const void* xs, int64_t rows_cap, int64_
     if (pair) {
         MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_pair_kernel<TIN, TIN, true>, c.device));
         LaunchScope scope(m, s, "tc_gate_up");
-        MUMMU_CUDA_TRY(launch_chain(chain_early(m), grouped_gemm_pair_kernel<TIN, TIN, true>, dim3(sms & ~1), (unsigned)(TC_THREADS), smem_pair, s, map_x, map_g, map_u, g));
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m, rows_est), grouped_gemm_pair_kernel<TIN, TIN, true>, dim3(sms & ~1), (unsigned)(TC_THREADS), smem_pair, s, map_x, map_g, map_u, g));
         MUMMU_CUDA_TRY(cudaGetLastError());
     } else {
         MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_tc_kernel<TIN, TIN, true>, c.device));
         LaunchScope scope(m, s, "tc_gate_up");
-        MUMMU_CUDA_TRY(launch_chain(chain_early(m), grouped_gemm_tc_kernel<TIN, TIN, true>, dim3(sms), (unsigned)(TC_THREADS), smem, s, map_x, map_g, map_u, g));
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m, rows_est), grouped_gemm_tc_kernel<TIN, TIN, true>, dim3(sms), (unsigned)(TC_THREADS), smem, s, map_x, map_g, map_u, g));
         MUMMU_CUDA_TRY(cudaGetLastError());
     }
     TcArgs d{};
@@ -700,13 +700,13 @@ static int launch_tc_typed(MummuMoe* m, const void* xs, int64_t rows_cap, int64_
     LaunchScope scope(m, s, "tc_down");
     if (pair && ys_dtype != MUMMU_F32) {
         MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_pair_kernel<TIN, TIN, false>, c.device));
-        MUMMU_CUDA_TRY(launch_chain(chain_early(m), grouped_gemm_pair_kernel<TIN, TIN, false>, dim3(sms & ~1), (unsigned)(TC_THREADS), smem_pair, s, map_h, map_d, map_d, d));
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m, rows_est), grouped_gemm_pair_kernel<TIN, TIN, false>, dim3(sms & ~1), (unsigned)(TC_THREADS), smem_pair, s, map_h, map_d, map_d, d));
     } else if (ys_dtype == MUMMU_F32) {
         MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_tc_kernel<TIN, float, false>, c.device));
-        MUMMU_CUDA_TRY(launch_chain(chain_early(m), grouped_gemm_tc_kernel<TIN, float, false>, dim3(sms), (unsigned)(TC_THREADS), smem, s, map_h, map_d, map_d, d));
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m, rows_est), grouped_gemm_tc_kernel<TIN, float, false>, dim3(sms), (unsigned)(TC_THREADS), smem, s, map_h, map_d, map_d, d));
     } else {
         MUMMU_CUDA_TRY(allow_big_smem(grouped_gemm_tc_kernel<TIN, TIN, false>, c.device));
-        MUMMU_CUDA_TRY(launch_chain(chain_early(m), grouped_gemm_tc_kernel<TIN, TIN, false>, dim3(sms), (unsigned)(TC_THREADS), smem, s, map_h, map_d, map_d, d));
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m, rows_est), grouped_gemm_tc_kernel<TIN, TIN, false>, dim3(sms), (unsigned)(TC_THREADS), smem, s, map_h, map_d, map_d, d));
     }
     MUMMU_CUDA_TRY(cudaGetLastError());
     return MUMMU_OK;
@@ -821,7 +821,7 @@ int launch_experts_q4k_tc(MummuMoe* m, const void* xs, int64_t rows_cap, int64_t
         }
         const int blocks_per_expert = (int)((int64_t)c.inter * c.hidden / 256);
         const dim3 grid((unsigned)((blocks_per_expert + QE_PER_CTA - 1) / QE_PER_CTA), (unsigned)c.experts_local, 3);
-        MUMMU_CUDA_TRY(launch_chain(chain_early(m), q4k_expand_f16_kernel, dim3(grid), (unsigned)(256), 0, s, eb, blocks_per_expert, counts));
+        MUMMU_CUDA_TRY(launch_chain(chain_early(m, rows_est), q4k_expand_f16_kernel, dim3(grid), (unsigned)(256), 0, s, eb, blocks_per_expert, counts));
         MUMMU_CUDA_TRY(cudaGetLastError());
     }
     const void* banks[3] = {owner->wexp[0], owner->wexp[1], owner->wexp[2]};
@@ -834,7 +834,7 @@ int launch_gather_rows(MummuMoe* m, const void* x, const int32_t* row_token, voi
     const int vec = m->cfg.hidden * 2 / 16;
     int64_t blocks = rows < 8 ? 1 : (rows / 8 < 148 * 8 ? (rows + 7) / 8 : 148 * 8);     // a warp per row
     LaunchScope scope(m, s, "gather_rows");
-    MUMMU_CUDA_TRY(launch_chain(chain_early(m), gather_rows_kernel, dim3((unsigned)blocks), (unsigned)(256), 0, s, (const uint4*)x, row_token, (uint4*)xs, rows, vec));
+    MUMMU_CUDA_TRY(launch_chain(chain_early(m, rows), gather_rows_kernel, dim3((unsigned)blocks), (unsigned)(256), 0, s, (const uint4*)x, row_token, (uint4*)xs, rows, vec));
     MUMMU_CUDA_TRY(cudaGetLastError());
     return MUMMU_OK;
 }
